@@ -15,15 +15,15 @@
 //
 // Design here: one persistent kernel per pass and path; each warp repeatedly
 // takes a work unit from a device counter — 32 TRA particles (one per lane) or
-// one 32-particle SMS task (candidates staged in batches in shared memory,
-// evaluated two at a time with packed FP32x2 arithmetic by every lane). The
-// grid is sized from the SM count, so the launch needs neither the host-side
-// TRA/SMS counts nor a host synchronisation. Neighbour rows merge the three
-// x-adjacent cells of each (dy, dz) row into one contiguous index range,
-// pruned by micro-x slab as in the reference (SMS rows at dz = -1 / +1 are
-// further cut to the micro-z groups that reach the task). Candidates are
-// visited rows z-major, then in increasing sorted index; the TRA density pass
-// records which interact as bit masks that the TRA force pass walks.
+// a cluster of 16 particles of an SMS task (candidates pruned by the cluster's
+// bounding box, staged in batches in shared memory and evaluated two at a time
+// with packed FP32x2 arithmetic). The grid is sized from the SM count, so the
+// launch needs neither the host-side TRA/SMS counts nor a host
+// synchronisation. TRA neighbour rows merge the three x-adjacent cells of each
+// (dy, dz) row into one contiguous index range, pruned by micro-x slab as in
+// the reference. Candidates are visited rows z-major, then in increasing
+// sorted index; the TRA density pass records which interact as bit masks that
+// the TRA force pass walks.
 #include <algorithm>
 
 #include "gsph_internal.h"
@@ -319,9 +319,6 @@ constexpr size_t kRowPrefetchCellBytes = size_t(64) << 20;
 // kernel is also built for 4 (gsph_tuning.warps_per_block), with twice the
 // CTAs per SM for the same occupancy.
 constexpr int kWarpsPerBlock = 8;
-// SMS candidates staged per batch (two per lane).
-constexpr int kSmsBatch = 64;
-constexpr int kDenBatch = 256;   // SMS density: candidates staged per batch
 // Coordinate of padding candidates: far outside any kernel radius.
 constexpr float kFar = 1.0e18f;
 
@@ -407,148 +404,254 @@ k_density_tra(Frame f, DevParams P) {
 }
 
 // ------------------------------------------------------- SMS candidates --
-// The candidates of an SMS task, row by row (rows z-major as in the
-// reference), each row in increasing sorted index. Rows at dz = 0 are the
-// reference's x-merged range (micro-x slabs pruned by the task's x bounds,
-// kernel_common.cuh:614-674). Rows at dz = -1 / +1 are further pruned in z: a
-// particle of the cell below (above) whose micro-z is below (above) every
-// task particle's own micro-z is at least h away from all of them, so only
-// the micro-z groups [zmin, 3] ([0, zmax]) of each micro-x slab are kept,
-// using the per-cell (micro-x, micro-z) group offsets of the sort. Pruned
-// candidates never interact, so the interacting set and its order are the
-// same as the reference's.
+// An SMS task's 32 particles are taken as clusters of C consecutive ones. A
+// warp works on one cluster: lane = (group g = lane / C, particle i = lane %
+// C), and the 32 / C groups share the cluster's candidates between them.
+// Consecutive particles of a cell lie close together (the sort order is
+// micro-x, micro-z, micro-y), so a small cluster's bounding box is small and
+// most candidates within h of the box interact with a given particle of it:
+// in the default scene (spacing 0.15 h, 1,237 neighbours per particle) 70 /
+// 56 / 46 / 40% for clusters of 4 / 8 / 16 / 32, of 1,764 / 2,197 / 2,693 /
+// 3,127 listed out of 4,155 / 4,481 / 4,861 / 5,343 tested. The pair
+// arithmetic is bound by the FP32 pipe and wants small clusters, the testing
+// by issue slots and wants large ones, and small scenes want many units:
+// force, 3.94M particles 14.0 / 12.5 ms and 64,000 particles 260 / 277 us at
+// C = 8 / 16; density 6.8 / 5.2 / 4.8 ms and 146 / 154 / 165 us at 8 / 16 /
+// 32. Whole tasks without the box test took 16.3 ms and 690 us (force), 6.7
+// ms and 230 us (density).
 //
-// Segment of lane l (< 12) of row cell m: cell m - 1 + l / 4, micro-x slab
-// l % 4, micro-z groups [zlo, zhi]; empty where the slab is outside the
-// task's x bounds or the cell outside the grid. A cell whose groups are
-// unknown (> 65,535 particles) is taken whole by its first lane.
-__device__ __forceinline__ void sms_segment(const Frame &f, const SceneGeom &G, int m,
-                                            int cx, int xlo, int xhi, int zlo,
-                                            int zhi, int lane, int &sb, int &sl) {
-    sb = 0;
-    sl = 0;
-    if (lane >= 12) return;
-    const int k = lane >> 2, mx = lane & 3;
-    if (k == 0 && (cx == 0 || mx < xlo)) return;
-    if (k == 2 && (cx + 1 >= G.gx || mx > xhi)) return;
-    const int c = m + k - 1;
-    const int cs = f.cell_start[c];
-    const int cnt = f.cell_start[c + 1] - cs;
-    if (cnt <= 0) return;
-    const uint16_t *g = f.cell_grp + size_t(c) * 16;
-    int b, e;
-    if (g[0] == kGroupsUnknown) {
-        if (mx != (k == 0 ? xlo : 0)) return;
-        b = k == 0 ? slab_begin(f, c, cs, cs + cnt, xlo) - cs : 0;
-        e = k == 2 ? slab_end(f, c, cs, cs + cnt, xhi) - cs : cnt;
-    } else {
-        b = g[mx * 4 + zlo];
-        e = zhi < 3 ? g[mx * 4 + zhi + 1] : (mx < 3 ? g[mx * 4 + 4] : cnt);
-        b = min(b, cnt);
-        e = min(e, cnt);
-    }
-    if (e > b) {
-        sb = cs + b;
-        sl = e - b;
-    }
+// Candidates are pruned twice before a pair is evaluated:
+//  * by micro cells: micro-x slab s of a neighbour cell keeps only the
+//    micro-z groups whose gap to the cluster's own micro cells, gx, gy, gz in
+//    quarters of h (gy of the whole cell), has gx^2 + gy^2 + gz^2 < 16: a
+//    particle beyond that is at least h away;
+//  * by the box: a candidate is listed only if its distance from the
+//    cluster's bounding box is at most h.
+// Both leave every interacting candidate in, in increasing sorted index per
+// row, rows z-major as in the reference.
+struct ClusterBox {
+    float cx, cy, cz, ex, ey, ez;       // a point inside, half extents from it
+    int x0, x1, y0, y1, z0, z1;         // micro cells inside the cell, [0, 3]
+};
+
+__device__ __forceinline__ float warp_max(float v) {   // v >= 0
+    return __uint_as_float(__reduce_max_sync(kFull, __float_as_uint(v)));
 }
 
-// Streams a task's candidates through a warp's kDenBatch-slot staging batch:
-// stage(slot, index) fills one slot, run(pairs) evaluates the staged slots
-// two at a time; batches run full except the last (its odd slot is padded
-// by pad(slot)). Control flow is warp-uniform.
-template <class Stage, class Pad, class Run>
-__device__ __forceinline__ void sms_stream(const Frame &f, const SceneGeom &G,
-                                           const gsph_block_task &task, int zmin,
-                                           int zmax, int lane, Stage stage, Pad pad,
-                                           Run run) {
-    const int cx = task.cell_pos[0], cy = task.cell_pos[1], cz = task.cell_pos[2];
-    int fill = 0;
-    auto take_range = [&](int b, int len) {
-        int o = 0;
-        while (o < len) {
-            const int n = min(len - o, kDenBatch - fill);
-            for (int t = lane; t < n; t += 32) stage(fill + t, b + o + t);
-            fill += n;
-            o += n;
-            if (fill == kDenBatch) {
-                __syncwarp();
-                run(kDenBatch / 2);
-                __syncwarp();
-                fill = 0;
+__device__ __forceinline__ ClusterBox cluster_box(const float4 &p, uint32_t key) {
+    ClusterBox b;
+    float l[3] = {p.x, p.y, p.z}, h[3] = {p.x, p.y, p.z};
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            l[a] = fminf(l[a], __shfl_xor_sync(kFull, l[a], o));
+            h[a] = fmaxf(h[a], __shfl_xor_sync(kFull, h[a], o));
+        }
+    b.cx = 0.5f * (l[0] + h[0]);
+    b.cy = 0.5f * (l[1] + h[1]);
+    b.cz = 0.5f * (l[2] + h[2]);
+    b.ex = warp_max(fabsf(p.x - b.cx));
+    b.ey = warp_max(fabsf(p.y - b.cy));
+    b.ez = warp_max(fabsf(p.z - b.cz));
+    const uint32_t m = __reduce_or_sync(kFull, (1u << ((key >> 4) & 3u)) |
+                                                   (16u << (key & 3u)) |
+                                                   (256u << ((key >> 2) & 3u)));
+    const uint32_t mx = m & 15u, my = (m >> 4) & 15u, mz = m >> 8;
+    b.x0 = __ffs(mx) - 1;
+    b.x1 = 31 - __clz(mx);
+    b.y0 = __ffs(my) - 1;
+    b.y1 = 31 - __clz(my);
+    b.z0 = __ffs(mz) - 1;
+    b.z1 = 31 - __clz(mz);
+    return b;
+}
+
+// Shared memory of one warp's candidate stream.
+constexpr int kSegMax = 27 * 4;    // a segment per neighbour cell and micro-x slab
+constexpr int kBatch = 128;        // candidates staged and evaluated at a time
+struct __align__(16) ClusterLists {
+    int2 seg[kSegMax];             // candidate ranges [x, y)
+    int idx[kBatch + 64];          // listed candidates
+};
+static_assert(kBatch % 64 == 0, "whole pairs per lane");
+
+// The candidate ranges of a cluster after the micro-cell pruning, one
+// neighbour cell per lane (27 of 32); returns their number.
+__device__ __forceinline__ int cluster_segments(const Frame &f, const SceneGeom &G,
+                                                const gsph_block_task &task,
+                                                const ClusterBox &b, int lane,
+                                                int2 *__restrict__ seg) {
+    const int dx = lane % 3 - 1, dy = lane / 3 % 3 - 1, dz = lane / 9 - 1;
+    const int x = task.cell_pos[0] + dx, y = task.cell_pos[1] + dy, z = task.cell_pos[2] + dz;
+    int2 own[4];
+    int n = 0;
+    if (lane < 27 && x >= 0 && x < G.gx && y >= 0 && y < G.gy && z >= 0 && z < G.gz) {
+        const int c = G.cbase + x + G.gx * (y + G.gy * z);
+        const int cs = f.cell_start[c];
+        const int cnt = f.cell_start[c + 1] - cs;
+        if (cnt > 0) {
+            const uint16_t *g = f.cell_grp + size_t(c) * 16;
+            const int gy = dy < 0 ? b.y0 : dy > 0 ? 3 - b.y1 : 0;
+            if (g[0] == kGroupsUnknown) {   // > 65,535 particles: taken whole
+                own[0] = make_int2(cs, cs + cnt);
+                n = 1;
+            } else {
+#pragma unroll
+                for (int s = 0; s < 4; ++s) {
+                    const int rx = 4 * dx + s;
+                    const int gx = max(0, max(rx - b.x1, b.x0 - rx) - 1);
+                    const int room = 15 - gx * gx - gy * gy;   // gz^2 <= room
+                    const int gz = room >= 9 ? 3 : room >= 4 ? 2 : room >= 1 ? 1 : 0;
+                    const int zlo = max(0, b.z0 - 1 - gz - 4 * dz);
+                    const int zhi = min(3, b.z1 + 1 + gz - 4 * dz);
+                    const bool some = room >= 0 && zlo <= zhi;
+                    const int lo = min(4 * s + zlo, 15), hi = 4 * s + zhi + 1;
+                    const int first = cs + min(some ? int(g[lo]) : 0, cnt);
+                    const int last =
+                        cs + (some ? (hi < 16 ? min(int(g[max(hi, 0)]), cnt) : cnt) : 0);
+                    own[s] = make_int2(first, some ? last : first);
+                }
+                // slabs that continue one another become one range
+                int m = 0;
+#pragma unroll
+                for (int s = 0; s < 4; ++s) {
+                    const int2 v = own[s];
+                    if (v.y <= v.x) continue;
+                    if (m > 0 && own[0].y == v.x && m == 1) {
+                        own[0].y = v.y;
+                    } else if (m > 1 && own[1].y == v.x && m == 2) {
+                        own[1].y = v.y;
+                    } else if (m > 2 && own[2].y == v.x && m == 3) {
+                        own[2].y = v.y;
+                    } else {
+                        if (m == 0) own[0] = v;
+                        if (m == 1) own[1] = v;
+                        if (m == 2) own[2] = v;
+                        if (m == 3) own[3] = v;
+                        ++m;
+                    }
+                }
+                n = m;
             }
         }
+    }
+    int incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += v;
+    }
+    const int at = incl - n;
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+        if (s < n) seg[at + s] = own[s];
+    __syncwarp();
+    return __shfl_sync(kFull, incl, 31);
+}
+
+// Streams a cluster's candidates: two runs of 32 positions are loaded
+// together and tested against the box (one candidate per lane), the indices
+// that pass are compacted into a list, and kBatch of them at a time are
+// staged and evaluated. fill(k, a, b) stages the pair k (one pair per lane, so
+// that the gathers are dense and in flight together) from the indices a and
+// b, where -1 stands for a candidate that interacts with nothing; run(n)
+// takes the first n * (32 / C) pairs, each group every (32 / C)-th of them.
+// Control flow is warp-uniform.
+template <int C, class Fill, class Run>
+__device__ __forceinline__ void cluster_stream(const Frame &f, const SceneGeom &G,
+                                               const gsph_block_task &task,
+                                               const ClusterBox &box, float h2, int lane,
+                                               ClusterLists &ls, Fill fill, Run run) {
+    constexpr int kStep = 2 * (32 / C);   // candidates per iteration of run
+    static_assert(kBatch % kStep == 0, "a batch is whole iterations");
+    const int nseg = cluster_segments(f, G, task, box, lane, ls.seg);
+    const unsigned lt = lanemask_lt();
+    // differences of coordinates round to 2^-24 of themselves, so 1e-5 of h^2
+    // covers the test's rounding
+    const float reach = h2 * 1.00001f;
+    auto near = [&](const float4 &q) {
+        const float ax = fmaxf(fabsf(q.x - box.cx) - box.ex, 0.f);
+        const float ay = fmaxf(fabsf(q.y - box.cy) - box.ey, 0.f);
+        const float az = fmaxf(fabsf(q.z - box.cz) - box.ez, 0.f);
+        return sq_dist(ax, ay, az) <= reach;
     };
-    for (int r = 0; r < 9; ++r) {
-        const int ny = cy + (r % 3) - 1;
-        const int nz = cz + (r / 3) - 1;
-        if (ny < 0 || ny >= G.gy || nz < 0 || nz >= G.gz) continue;
-        const int m = G.cbase + cx + G.gx * (ny + G.gy * nz);
-        const int dz = r / 3 - 1;
-        const int zlo = dz < 0 ? zmin : 0, zhi = dz > 0 ? zmax : 3;
-        if ((zlo == 0 && zhi == 3) || !f.cell_grp) {
-            int begin, end;
-            row_range(f, G, m, cx, task.xxi, task.xxx, begin, end);
-            take_range(begin, end - begin);
-        } else {
-            int sb, sl;
-            sms_segment(f, G, m, cx, task.xxi, task.xxx, zlo, zhi, lane, sb, sl);
-            const unsigned nonempty = __ballot_sync(kFull, sl > 0);
-            for (unsigned w = nonempty; w; w &= w - 1) {
-                const int src = __ffs(w) - 1;
-                take_range(__shfl_sync(kFull, sb, src), __shfl_sync(kFull, sl, src));
+    int cnt = 0;
+    auto batch = [&](int n) {   // stage and evaluate the first n listed
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < kBatch / 2; q += 32) {
+            const int2 ab = *reinterpret_cast<const int2 *>(ls.idx + 2 * (q + lane));
+            fill(q + lane, 2 * (q + lane) < n ? ab.x : -1, 2 * (q + lane) + 1 < n ? ab.y : -1);
+        }
+        __syncwarp();
+        run((n + kStep - 1) / kStep);
+        __syncwarp();
+    };
+    for (int k = 0; k < nseg; ++k) {
+        const int2 sg = ls.seg[k];
+        for (int j0 = sg.x; j0 < sg.y; j0 += 64) {
+            const int ja = j0 + lane, jb = ja + 32;
+            const float4 qa = f.pos[min(ja, sg.y - 1)];
+            const float4 qb = f.pos[min(jb, sg.y - 1)];
+            const bool ina = ja < sg.y && near(qa);
+            const bool inb = jb < sg.y && near(qb);
+            const unsigned ha = __ballot_sync(kFull, ina);
+            const unsigned hb = __ballot_sync(kFull, inb);
+            const int na = cnt + __popc(ha);
+            if (ina) ls.idx[cnt + __popc(ha & lt)] = ja;
+            if (inb) ls.idx[na + __popc(hb & lt)] = jb;
+            cnt = na + __popc(hb);
+            if (cnt >= kBatch) {
+                batch(kBatch);
+                cnt -= kBatch;   // at most 63 stay
+                int v0 = 0, v1 = 0;
+                if (lane < cnt) v0 = ls.idx[kBatch + lane];
+                if (lane + 32 < cnt) v1 = ls.idx[kBatch + lane + 32];
+                __syncwarp();
+                if (lane < cnt) ls.idx[lane] = v0;
+                if (lane + 32 < cnt) ls.idx[lane + 32] = v1;
             }
         }
     }
-    if (fill > 0) {
-        if ((fill & 1) && lane == 0) pad(fill);
-        __syncwarp();
-        run((fill + 1) >> 1);
-        __syncwarp();
-    }
-}
-
-// Micro-z range of a task's particles (warp-wide; inactive lanes neutral).
-__device__ __forceinline__ void task_z_range(const Frame &f, int self, bool active,
-                                             int &zmin, int &zmax) {
-    const int mz = active ? int((f.key[self] >> 2) & 3u) : -1;
-    zmin = int(__reduce_min_sync(kFull, unsigned(active ? mz : 3)));
-    zmax = __reduce_max_sync(kFull, active ? mz : 0);
+    if (cnt > 0) batch(cnt);
+    __syncwarp();
 }
 
 // ------------------------------------------------------------ density SMS --
-// One 32-particle task per warp (density_kernels.cu:368-565). Candidates are
-// streamed 256 at a time into shared memory, each pair (slots 2k, 2k+1) as an
-// (x, x, y, y) float4 and a (z, z) float2; every lane evaluates them two at a
-// time with packed FP32x2 arithmetic and the TRA pass's one-compare cut-off
-// test.
+// One cluster of kDenCluster particles per warp (density_kernels.cu:368-565).
+// Bound by issue slots, more than half of them in the candidate tests.
+// Candidates are staged as pairs (slots 2k, 2k+1), an (x, x, y, y) float4 and
+// a (z, z) float2, and evaluated two at a time with packed FP32x2 arithmetic
+// and the TRA pass's one-compare cut-off test; the groups' sums are added at
+// the end.
+constexpr int kDenCluster = 16;
 template <int W>
 __global__ void __launch_bounds__(W * 32, 4 * kWarpsPerBlock / W)
 k_density_sms(Frame f, DevParams P) {
+    constexpr int C = kDenCluster, kGroups = 32 / C;
     // candidate pair k (slots 2k, 2k+1): (x, x, y, y) and (z, z)
-    __shared__ __align__(16) float4 sms_xy[W][kDenBatch / 2];
-    __shared__ __align__(16) float2 sms_zz[W][kDenBatch / 2];
+    __shared__ __align__(16) float4 sms_xy[W][kBatch / 2];
+    __shared__ __align__(16) float2 sms_zz[W][kBatch / 2];
+    __shared__ ClusterLists lists[W];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int task_count = f.ctr->task_count;
     if (task_count == 0) return;   // no SMS work: skip the queue atomics
-    float *fxy = reinterpret_cast<float *>(sms_xy[warp]);
-    float *fz = reinterpret_cast<float *>(sms_zz[warp]);
-    const float4 *sxy = sms_xy[warp];
-    const float2 *szz = sms_zz[warp];
+    float4 *sxy = sms_xy[warp];
+    float2 *szz = sms_zz[warp];
+    const int i = lane % C, g = lane / C;
     for (;;) {
         const int u = next_unit(&f.ctr->work_density_sms);
-        if (u >= task_count) break;
-        const gsph_block_task task = f.tasks[u];
-        const int cb = task.cell_begin;
-        const int cend = cb + task.cell_particle_count;
-        const int self = cb + task_offset(task) + lane;
-        const bool active = self < cend;
-        if (cb + task_offset(task) >= cend) continue;   // warp-uniform
-        const float4 p = f.pos[active ? self : cend - 1];
+        if (u / kGroups >= task_count) break;
+        const gsph_block_task task = f.tasks[u / kGroups];
+        const int first = task.cell_begin + task_offset(task) + (u % kGroups) * C;
+        const int cend = task.cell_begin + task.cell_particle_count;
+        if (first >= cend) continue;   // warp-uniform
+        const int self = min(first + i, cend - 1);
+        const float4 p = f.pos[self];
         const SceneGeom G = geom_of_cell(f.scenes, task.cellid);
-        int zmin, zmax;
-        task_z_range(f, self, active, zmin, zmax);
+        const ClusterBox box = cluster_box(p, f.key[self]);
         const float2 npx = make_float2(-p.x, -p.x);
         const float2 npy = make_float2(-p.y, -p.y);
         const float2 npz = make_float2(-p.z, -p.z);
@@ -558,28 +661,22 @@ k_density_sms(Frame f, DevParams P) {
         const float2 msm = make_float2(-kFloatSmall, -kFloatSmall);
         const float2 m1 = make_float2(-1.f, -1.f);
         float2 acc = make_float2(0.f, 0.f);
-        sms_stream(
-            f, G, task, zmin, zmax, lane,
-            [&](int slot, int j) {
-                const float4 q = f.pos[j];
-                const int o = (slot >> 1) * 4 + (slot & 1);
-                fxy[o] = q.x;
-                fxy[o + 2] = q.y;
-                fz[slot] = q.z;
+        const float4 far = make_float4(kFar, kFar, kFar, 0.f);
+        cluster_stream<C>(
+            f, G, task, box, P.h2, lane, lists[warp],
+            [&](int k, int ja, int jb) {
+                const float4 a = ja < 0 ? far : f.pos[ja];
+                const float4 b = jb < 0 ? far : f.pos[jb];
+                sxy[k] = make_float4(a.x, b.x, a.y, b.y);
+                szz[k] = make_float2(a.z, b.z);
             },
-            [&](int slot) {
-                const int o = (slot >> 1) * 4 + (slot & 1);
-                fxy[o] = kFar;
-                fxy[o + 2] = kFar;
-                fz[slot] = kFar;
-            },
-            [&](int pairs) {
-#pragma unroll 32
-                for (int k = 0; k < pairs; ++k) {
-                    const float4 qa = sxy[k];
+            [&](int n) {
+#pragma unroll 8
+                for (int k = 0; k < n; ++k) {
+                    const float4 qa = sxy[k * kGroups + g];
                     const float2 dx = __fadd2_rn(make_float2(qa.x, qa.y), npx);
                     const float2 dy = __fadd2_rn(make_float2(qa.z, qa.w), npy);
-                    const float2 dz = __fadd2_rn(szz[k], npz);
+                    const float2 dz = __fadd2_rn(szz[k * kGroups + g], npz);
                     // the cut-off test of sq_dist_less_small, per half
                     float2 e = __ffma2_rn(dx, dx, msm);
                     e = __ffma2_rn(dy, dy, e);
@@ -590,7 +687,10 @@ k_density_sms(Frame f, DevParams P) {
                     acc = __ffma2_rn(__fmul2_rn(t, t), t, acc);
                 }
             });
-        if (active) write_density(f, P, self, acc.x + acc.y, true);
+        float sum = acc.x + acc.y;
+#pragma unroll
+        for (int o = C; o < 32; o <<= 1) sum += __shfl_xor_sync(kFull, sum, o);
+        if (g == 0 && first + i < cend) write_density(f, P, self, sum, true);
     }
 }
 
@@ -701,49 +801,54 @@ k_force_tra(Frame f, DevParams P, bool fresh) {
 }
 
 // -------------------------------------------------------------- force SMS --
-// One 32-particle task per warp (force_kernels.cu:830-1054). The candidates
-// are the density pass's: x-merged rows, those at dz = -1 / +1 cut to the
-// micro-z groups that can reach the task, one (cell, micro-x slab) segment at
-// a time. They are staged 64 at a time in shared memory, each candidate pair
-// as four float4s (one 16-byte broadcast load per pair and quantity group),
-// and evaluated two at a time with packed FP32x2 arithmetic; a pair is
-// skipped when no lane of the warp interacts with either candidate. Each
-// term rounds as the reference's scalar expression; the two halves of every
-// accumulator are summed at the end.
+// One cluster of kForceCluster particles per warp (force_kernels.cu:830-1054),
+// over the density pass's candidates. Bound by the FP32 pipe (61% busy; 28 of
+// the 43 instructions of a pair step are packed) and, beside it, by the
+// candidate tests. Three blocks per SM: at four, 64 registers spill inside the
+// pair loop (3.94M particles 13.3 ms against 12.5). Each candidate pair is staged as four
+// float4s (one 16-byte load per pair and quantity group) and evaluated with
+// packed FP32x2 arithmetic. Each term rounds as the reference's scalar
+// expression; the two halves of every accumulator and then the groups' sums
+// are added at the end.
+constexpr int kForceCluster = 16;
+constexpr int kForceSmsCtas = 3;   // resident blocks per SM
 template <bool kArt, int W>
-__global__ void __launch_bounds__(W * 32, 4 * kWarpsPerBlock / W)
+__global__ void __launch_bounds__(W * 32, kForceSmsCtas * kWarpsPerBlock / W)
 k_force_sms(Frame f, DevParams P) {
+    constexpr int C = kForceCluster, kGroups = 32 / C;
     // candidate pair k (slots 2k, 2k+1) as four float4s: (x, x, y, y),
     // (z, z, 1/rho, 1/rho), (vx, vx, vy, vy), (vz, vz, p, p)
-    __shared__ __align__(16) float4 sm[4][W][kSmsBatch / 2];
+    __shared__ __align__(16) float4 sm[4][W][kBatch / 2];
+    __shared__ ClusterLists lists[W];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int task_count = f.ctr->task_count;
     if (task_count == 0) return;   // no SMS work: skip the queue atomics
     float4 *sa = sm[0][warp], *sb4 = sm[1][warp], *sc = sm[2][warp], *sd = sm[3][warp];
+    const int i = lane % C, g = lane / C;
     for (;;) {
         const int u = next_unit(&f.ctr->work_force_sms);
-        if (u >= task_count) break;
-        const gsph_block_task task = f.tasks[u];
-        const int cb = task.cell_begin;
-        const int cend = cb + task.cell_particle_count;
-        const int self = cb + task_offset(task) + lane;
-        const bool active = self < cend;
-        if (cb + task_offset(task) >= cend) continue;
-        const int safe = active ? self : cend - 1;
-        const float4 p = f.pos[safe];
-        const float4 pev = f.ev[safe];
+        if (u / kGroups >= task_count) break;
+        const gsph_block_task task = f.tasks[u / kGroups];
+        const int first = task.cell_begin + task_offset(task) + (u % kGroups) * C;
+        const int cend = task.cell_begin + task.cell_particle_count;
+        if (first >= cend) continue;   // warp-uniform
+        const int self = min(first + i, cend - 1);
+        const float4 p = f.pos[self];
+        const float4 pev = f.ev[self];
         const SceneGeom G = geom_of_cell(f.scenes, task.cellid);
-        const int cx = task.cell_pos[0], cy = task.cell_pos[1],
-                  cz = task.cell_pos[2];
+        const ClusterBox box = cluster_box(p, f.key[self]);
         const float2 npx = make_float2(-p.x, -p.x);
         const float2 npy = make_float2(-p.y, -p.y);
         const float2 npz = make_float2(-p.z, -p.z);
-        const float2 nvx = make_float2(-pev.x, -pev.x);
-        const float2 nvy = make_float2(-pev.y, -pev.y);
-        const float2 nvz = make_float2(-pev.z, -pev.z);
-        int zmin, zmax;
-        task_z_range(f, self, active, zmin, zmax);
+        // velocities relative to the cluster's first particle: the viscosity
+        // sum of V_j (v_j - v_i)(h - r) is then taken as the sum of V_j v_j
+        // (h - r) less v_i times the sum of V_j (h - r), two packed
+        // operations less per pair, without losing the small differences
+        const float ux = __shfl_sync(kFull, pev.x, 0);
+        const float uy = __shfl_sync(kFull, pev.y, 0);
+        const float uz = __shfl_sync(kFull, pev.z, 0);
+        const float wx = pev.x - ux, wy = pev.y - uy, wz = pev.z - uz;
         const float2 pi2 = make_float2(pev.w, pev.w);
         const float2 h2v = make_float2(P.h2, P.h2);
         const float2 hv = make_float2(P.h, P.h);
@@ -753,118 +858,100 @@ k_force_sms(Frame f, DevParams P) {
         // pressure sum gets -r*ps = d*ps with d = q - p; the colour
         // gradient is accumulated with the opposite sign and negated at the end
         float2 Px = zero, Py = zero, Pz = zero, Vx = zero, Vy = zero, Vz = zero;
-        float2 Gx = zero, Gy = zero, Gz = zero, L = zero;
-        for (int r = 0; r < 9; ++r) {
-            const int ny = cy + (r % 3) - 1;
-            const int nz = cz + (r / 3) - 1;
-            if (ny < 0 || ny >= G.gy || nz < 0 || nz >= G.gz) continue;
-            const int m = G.cbase + cx + G.gx * (ny + G.gy * nz);
-            // rows at dz = -1 / +1 keep only the micro-z groups that can
-            // reach the task (as the density pass's candidate stream)
-            const int rdz = r / 3 - 1;
-            const int zlo = rdz < 0 ? zmin : 0, zhi = rdz > 0 ? zmax : 3;
-            const bool zcut = f.cell_grp && !(zlo == 0 && zhi == 3);
-            int begin = 0, end = 0;
-            if (!zcut) row_range(f, G, m, cx, task.xxi, task.xxx, begin, end);
-            const int nseg = zcut ? 12 : 1;
-            for (int sg = 0; sg < nseg; ++sg) {
-                if (zcut) {
-                    int sb, sl;
-                    sms_segment(f, G, m, cx, task.xxi, task.xxx, zlo, zhi, sg, sb, sl);
-                    begin = sb;
-                    end = sb + sl;
+        float2 Gx = zero, Gy = zero, Gz = zero, L = zero, S = zero;
+        // added to r^2 so that 1/r stays finite for the particle itself, whose
+        // terms are zeroed; far below a rounding of any interacting r^2
+        const float2 tiny = make_float2(1e-30f, 1e-30f);
+        const float4 far = make_float4(kFar, kFar, kFar, 0.f);
+        const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+        cluster_stream<C>(
+            f, G, task, box, P.h2, lane, lists[warp],
+            [&](int k, int ja, int jb) {
+                const float4 a = ja < 0 ? far : f.pos[ja];
+                const float4 b = jb < 0 ? far : f.pos[jb];
+                const float4 va = ja < 0 ? none : f.ev[ja];
+                const float4 vb = jb < 0 ? none : f.ev[jb];
+                sa[k] = make_float4(a.x, b.x, a.y, b.y);
+                sb4[k] = make_float4(a.z, b.z, a.w, b.w);
+                sc[k] = make_float4(va.x - ux, vb.x - ux, va.y - uy, vb.y - uy);
+                sd[k] = make_float4(va.z - uz, vb.z - uz, va.w, vb.w);
+            },
+            [&](int n) {
+#pragma unroll 4
+                for (int k = 0; k < n; ++k) {
+                    const int s = k * kGroups + g;
+                    const float4 qa = sa[s], qb = sb4[s];
+                    const float2 dx = __fadd2_rn(make_float2(qa.x, qa.y), npx);
+                    const float2 dy = __fadd2_rn(make_float2(qa.z, qa.w), npy);
+                    const float2 dz = __fadd2_rn(make_float2(qb.x, qb.y), npz);
+                    float2 d2 = __ffma2_rn(dx, dx, tiny);
+                    d2 = __ffma2_rn(dy, dy, d2);
+                    d2 = __ffma2_rn(dz, dz, d2);
+                    const float2 t = __ffma2_rn(d2, m1, h2v);   // h^2 - r^2
+                    const bool okx = t.x >= 0.f && d2.x >= kFloatSmall;
+                    const bool oky = t.y >= 0.f && d2.y >= kFloatSmall;
+                    const float2 inv = make_float2(rsqrtf(d2.x), rsqrtf(d2.y));
+                    const float2 d = __fmul2_rn(d2, inv);
+                    const float2 kk = __ffma2_rn(d, m1, hv);       // h - r
+                    // 1/rho of the candidate, zero where it does not interact:
+                    // the pressure, viscosity and colour terms vanish with it
+                    const float2 V = make_float2(okx ? qb.z : 0.f, oky ? qb.w : 0.f);
+                    const float4 qc = sc[s], qd = sd[s];
+                    const float2 wk = __fmul2_rn(V, kk);
+                    const float2 psum = __fadd2_rn(pi2, make_float2(qd.z, qd.w));
+                    const float2 ps = __fmul2_rn(__fmul2_rn(__fmul2_rn(wk, psum), kk), inv);
+                    Px = __ffma2_rn(dx, ps, Px);
+                    Py = __ffma2_rn(dy, ps, Py);
+                    Pz = __ffma2_rn(dz, ps, Pz);
+                    if (kArt) {
+                        // v_ij . r_ij = (v_j - v_i) . (x_j - x_i); the sum is
+                        // kept against d = x_j - x_i and negated at the end
+                        const float2 dvx = __fadd2_rn(make_float2(qc.x, qc.y), make_float2(-wx, -wx));
+                        const float2 dvy = __fadd2_rn(make_float2(qc.z, qc.w), make_float2(-wy, -wy));
+                        const float2 dvz = __fadd2_rn(make_float2(qd.x, qd.y), make_float2(-wz, -wz));
+                        float2 vr = __fmul2_rn(dvx, dx);
+                        vr = __ffma2_rn(dvy, dy, vr);
+                        vr = __ffma2_rn(dvz, dz, vr);
+                        const float2 w = make_float2(
+                            okx ? artificial_pair(vr.x, d2.x, kk.x, inv.x, p.w, qb.z, P) : 0.f,
+                            oky ? artificial_pair(vr.y, d2.y, kk.y, inv.y, p.w, qb.w, P) : 0.f);
+                        Vx = __ffma2_rn(dx, w, Vx);
+                        Vy = __ffma2_rn(dy, w, Vy);
+                        Vz = __ffma2_rn(dz, w, Vz);
+                    } else {
+                        Vx = __ffma2_rn(make_float2(qc.x, qc.y), wk, Vx);
+                        Vy = __ffma2_rn(make_float2(qc.z, qc.w), wk, Vy);
+                        Vz = __ffma2_rn(make_float2(qd.x, qd.y), wk, Vz);
+                        S = __fadd2_rn(S, wk);
+                    }
+                    const float2 wh = __fmul2_rn(V, t);
+                    const float2 gw = __fmul2_rn(wh, t);
+                    Gx = __ffma2_rn(dx, gw, Gx);
+                    Gy = __ffma2_rn(dy, gw, Gy);
+                    Gz = __ffma2_rn(dz, gw, Gz);
+                    L = __ffma2_rn(wh, __ffma2_rn(t, m075, d2), L);
                 }
-                for (int base = begin; base < end; base += kSmsBatch) {
-                    const int cnt = min(kSmsBatch, end - base);
+            });
+        const float sw = S.x + S.y;
+        float s[10] = {Px.x + Px.y, Py.x + Py.y, Pz.x + Pz.y,
+                       Vx.x + Vx.y - wx * sw, Vy.x + Vy.y - wy * sw, Vz.x + Vz.y - wz * sw,
+                       Gx.x + Gx.y, Gy.x + Gy.y, Gz.x + Gz.y, L.x + L.y};
 #pragma unroll
-                    for (int hh = 0; hh < kSmsBatch; hh += 32) {
-                        const int t = hh + lane;
-                        float4 q = make_float4(kFar, kFar, kFar, 0.f);
-                        float4 qv = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (t < cnt) {
-                            q = f.pos[base + t];
-                            qv = f.ev[base + t];
-                        }
-                        const int o = (t >> 1) * 4 + (t & 1);
-                        float *fa = reinterpret_cast<float *>(sa), *fb = reinterpret_cast<float *>(sb4);
-                        float *fc = reinterpret_cast<float *>(sc), *fd = reinterpret_cast<float *>(sd);
-                        fa[o] = q.x; fa[o + 2] = q.y; fb[o] = q.z; fb[o + 2] = q.w;
-                        fc[o] = qv.x; fc[o + 2] = qv.y; fd[o] = qv.z; fd[o + 2] = qv.w;
-                    }
-                    __syncwarp();
-                    const int pairs = (cnt + 1) >> 1;
-#pragma unroll 8
-                    for (int k = 0; k < pairs; ++k) {
-                        const float4 qa = sa[k], qb = sb4[k];
-                        const float2 dx = __fadd2_rn(make_float2(qa.x, qa.y), npx);
-                        const float2 dy = __fadd2_rn(make_float2(qa.z, qa.w), npy);
-                        const float2 dz = __fadd2_rn(make_float2(qb.x, qb.y), npz);
-                        float2 d2 = __fmul2_rn(dx, dx);
-                        d2 = __ffma2_rn(dy, dy, d2);
-                        d2 = __ffma2_rn(dz, dz, d2);
-                        const float2 t = __ffma2_rn(d2, m1, h2v);   // h^2 - r^2
-                        const bool okx = t.x >= 0.f && d2.x >= kFloatSmall;
-                        const bool oky = t.y >= 0.f && d2.y >= kFloatSmall;
-                        if (!__any_sync(kFull, active && (okx || oky))) continue;
-                        const float2 d2s = make_float2(okx ? d2.x : 1.f, oky ? d2.y : 1.f);
-                        const float2 inv = make_float2(rsqrtf(d2s.x), rsqrtf(d2s.y));
-                        const float2 d = __fmul2_rn(d2s, inv);
-                        const float2 kk = __ffma2_rn(d, m1, hv);       // h - r
-                        // 1/rho of the candidate, zero where it does not interact:
-                        // the pressure, viscosity and colour terms vanish with it
-                        const float2 V = make_float2(okx ? qb.z : 0.f, oky ? qb.w : 0.f);
-                        const float4 qc = sc[k], qd = sd[k];
-                        const float2 wk = __fmul2_rn(V, kk);
-                        const float2 psum = __fadd2_rn(pi2, make_float2(qd.z, qd.w));
-                        const float2 ps = __fmul2_rn(__fmul2_rn(__fmul2_rn(wk, psum), kk), inv);
-                        Px = __ffma2_rn(dx, ps, Px);
-                        Py = __ffma2_rn(dy, ps, Py);
-                        Pz = __ffma2_rn(dz, ps, Pz);
-                        const float2 dvx = __fadd2_rn(make_float2(qc.x, qc.y), nvx);
-                        const float2 dvy = __fadd2_rn(make_float2(qc.z, qc.w), nvy);
-                        const float2 dvz = __fadd2_rn(make_float2(qd.x, qd.y), nvz);
-                        if (kArt) {
-                            // v_ij . r_ij = (v_j - v_i) . (x_j - x_i); the sum is
-                            // kept against d = x_j - x_i and negated at the end
-                            float2 vr = __fmul2_rn(dvx, dx);
-                            vr = __ffma2_rn(dvy, dy, vr);
-                            vr = __ffma2_rn(dvz, dz, vr);
-                            const float2 w = make_float2(
-                                okx ? artificial_pair(vr.x, d2s.x, kk.x, inv.x, p.w, qb.z, P)
-                                    : 0.f,
-                                oky ? artificial_pair(vr.y, d2s.y, kk.y, inv.y, p.w, qb.w, P)
-                                    : 0.f);
-                            Vx = __ffma2_rn(dx, w, Vx);
-                            Vy = __ffma2_rn(dy, w, Vy);
-                            Vz = __ffma2_rn(dz, w, Vz);
-                        } else {
-                            Vx = __ffma2_rn(dvx, wk, Vx);
-                            Vy = __ffma2_rn(dvy, wk, Vy);
-                            Vz = __ffma2_rn(dvz, wk, Vz);
-                        }
-                        const float2 wh = __fmul2_rn(V, t);
-                        const float2 gw = __fmul2_rn(wh, t);
-                        Gx = __ffma2_rn(dx, gw, Gx);
-                        Gy = __ffma2_rn(dy, gw, Gy);
-                        Gz = __ffma2_rn(dz, gw, Gz);
-                        L = __ffma2_rn(wh, __ffma2_rn(t, m075, d2), L);
-                    }
-                    __syncwarp();
-                }
-            }
-        }
-        if (active) {
+        for (int k = 0; k < 10; ++k)
+#pragma unroll
+            for (int o = C; o < 32; o <<= 1) s[k] += __shfl_xor_sync(kFull, s[k], o);
+        if (g == 0 && first + i < cend) {
             ForceAcc a;
-            a.px = Px.x + Px.y;
-            a.py = Py.x + Py.y;
-            a.pz = Pz.x + Pz.y;
-            a.vx = kArt ? -(Vx.x + Vx.y) : Vx.x + Vx.y;
-            a.vy = kArt ? -(Vy.x + Vy.y) : Vy.x + Vy.y;
-            a.vz = kArt ? -(Vz.x + Vz.y) : Vz.x + Vz.y;
-            a.gx = -(Gx.x + Gx.y);
-            a.gy = -(Gy.x + Gy.y);
-            a.gz = -(Gz.x + Gz.y);
-            a.lap = L.x + L.y;
+            a.px = s[0];
+            a.py = s[1];
+            a.pz = s[2];
+            a.vx = kArt ? -s[3] : s[3];
+            a.vy = kArt ? -s[4] : s[4];
+            a.vz = kArt ? -s[5] : s[5];
+            a.gx = -s[6];
+            a.gy = -s[7];
+            a.gz = -s[8];
+            a.lap = s[9];
             write_force(f, P, self, p, pev, G, a, true);
         }
     }
@@ -1048,9 +1135,9 @@ cudaError_t configure_shape(int smem) {
         return e;
     if ((e = set_carveout(k_force_tra<true, W>, kMaxShape.force_tra * k, smem, W * 32)))
         return e;
-    if ((e = set_carveout(k_force_sms<false, W>, kMaxShape.force_sms * k, smem, W * 32)))
+    if ((e = set_carveout(k_force_sms<false, W>, kForceSmsCtas * k, smem, W * 32)))
         return e;
-    return set_carveout(k_force_sms<true, W>, kMaxShape.force_sms * k, smem, W * 32);
+    return set_carveout(k_force_sms<true, W>, kForceSmsCtas * k, smem, W * 32);
 }
 
 template <int W>
