@@ -46,6 +46,17 @@ __device__ __forceinline__ float sq_dist(float dx, float dy, float dz) {
     return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
 }
 
+// a b + c d and a . b with one fixed rounding sequence. Where an expression
+// leaves the compiler a choice of which product to fuse, its choice may differ
+// between the builds of a kernel, and the builds have to give the same bits.
+__device__ __forceinline__ float mad2(float a, float b, float c, float d) {
+    return __fmaf_rn(a, b, __fmul_rn(c, d));
+}
+__device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, float by,
+                                      float bz) {
+    return __fmaf_rn(az, bz, mad2(ax, bx, ay, by));
+}
+
 // The TRA density pass's cut-off test in one unsigned compare: with
 // e = d^2 - kFloatSmall (the subtraction folded into the first fused
 // multiply-add), the reference's kFloatSmall <= d^2 <= h^2 is
@@ -157,7 +168,7 @@ __device__ __forceinline__ void force_pair(const float4 &self,
     a.py -= ry * ps;
     a.pz -= rz * ps;
     if (kArt) {
-        const float vr = (sev.x - qev.x) * rx + (sev.y - qev.y) * ry + (sev.z - qev.z) * rz;
+        const float vr = dot3(sev.x - qev.x, sev.y - qev.y, sev.z - qev.z, rx, ry, rz);
         const float w = artificial_pair(vr, d2, k, inv_d, self.w, V, P);
         a.vx += rx * w;
         a.vy += ry * w;
@@ -201,42 +212,42 @@ __device__ __forceinline__ void integrate_one(const float4 tp, const float4 v4,
     const float kernel = P.wall_kernel;
     float diff;
     diff = kernel - (tp.y - P.bmin);
-    if (diff > 0.0f) ay += alpha * diff - beta * vy;
+    if (diff > 0.0f) ay += mad2(alpha, diff, -beta, vy);
     diff = kernel - (G.bmax_y - tp.y);
-    if (diff > 0.0f) ay -= alpha * diff + beta * vy;
+    if (diff > 0.0f) ay -= mad2(alpha, diff, beta, vy);
     diff = kernel - (tp.x - P.bmin);
-    if (diff > 0.0f) ax += alpha * diff - beta * vx;
+    if (diff > 0.0f) ax += mad2(alpha, diff, -beta, vx);
     diff = kernel - (G.bmax_x - tp.x);
-    if (diff > 0.0f) ax -= alpha * diff + beta * vx;
+    if (diff > 0.0f) ax -= mad2(alpha, diff, beta, vx);
     diff = kernel - (tp.z - P.bmin);
-    if (diff > 0.0f) az += alpha * diff - beta * vz;
+    if (diff > 0.0f) az += mad2(alpha, diff, -beta, vz);
     diff = kernel - (G.bmax_z - tp.z);
-    if (diff > 0.0f) az -= alpha * diff + beta * vz;
+    if (diff > 0.0f) az -= mad2(alpha, diff, beta, vz);
     const float acc_limit = 3000000.f;
     const float vel_limit = 36.f;
-    ax = ax * tp.w + P.gx_acc;
-    ay = ay * tp.w + P.gy_acc;
-    az = az * tp.w + P.gz_acc;
-    float speed = ax * ax + ay * ay + az * az;
+    ax = __fmaf_rn(ax, tp.w, P.gx_acc);
+    ay = __fmaf_rn(ay, tp.w, P.gy_acc);
+    az = __fmaf_rn(az, tp.w, P.gz_acc);
+    float speed = dot3(ax, ay, az, ax, ay, az);
     if (speed > acc_limit) {
         const float s = sqrtf(acc_limit / speed);
         ax *= s;
         ay *= s;
         az *= s;
     }
-    vx += ax * P.time_step;
-    vy += ay * P.time_step;
-    vz += az * P.time_step;
-    speed = vx * vx + vy * vy + vz * vz;
+    vx = __fmaf_rn(ax, P.time_step, vx);
+    vy = __fmaf_rn(ay, P.time_step, vy);
+    vz = __fmaf_rn(az, P.time_step, vz);
+    speed = dot3(vx, vy, vz, vx, vy, vz);
     if (speed > vel_limit) {
         const float s = sqrtf(vel_limit / speed);
         vx *= s;
         vy *= s;
         vz *= s;
     }
-    float px = tp.x + vx * P.time_step;
-    float py = tp.y + vy * P.time_step;
-    float pz = tp.z + vz * P.time_step;
+    float px = __fmaf_rn(vx, P.time_step, tp.x);
+    float py = __fmaf_rn(vy, P.time_step, tp.y);
+    float pz = __fmaf_rn(vz, P.time_step, tp.z);
     if (px >= G.bmax_x) { vx *= P.wall_damping; px = G.bmax_x - kernel; }
     if (px <= P.bmin) { vx *= P.wall_damping; px = P.bmin + kernel; }
     if (py >= G.bmax_y) { vy *= P.wall_damping; py = G.bmax_y - kernel; }
@@ -258,13 +269,13 @@ __device__ __forceinline__ void write_force(const Frame &f, const DevParams &P,
     if (P.visc_artificial) {
         // -m rho_i sum Pi grad W: the mass is applied below with the rest
         const float c = -P.spiky * __fdividef(1.0f, p.w);
-        tx = a.px * P.half_spiky + a.vx * c;
-        ty = a.py * P.half_spiky + a.vy * c;
-        tz = a.pz * P.half_spiky + a.vz * c;
+        tx = mad2(a.px, P.half_spiky, a.vx, c);
+        ty = mad2(a.py, P.half_spiky, a.vy, c);
+        tz = mad2(a.pz, P.half_spiky, a.vz, c);
     } else {
-        tx = a.px * P.half_spiky + a.vx * P.visco_coef;
-        ty = a.py * P.half_spiky + a.vy * P.visco_coef;
-        tz = a.pz * P.half_spiky + a.vz * P.visco_coef;
+        tx = mad2(a.px, P.half_spiky, a.vx, P.visco_coef);
+        ty = mad2(a.py, P.half_spiky, a.vy, P.visco_coef);
+        tz = mad2(a.pz, P.half_spiky, a.vz, P.visco_coef);
     }
     const float gx = a.gx * P.grad_color_scale;
     const float gy = a.gy * P.grad_color_scale;
@@ -272,7 +283,7 @@ __device__ __forceinline__ void write_force(const Frame &f, const DevParams &P,
     float lap = a.lap * P.lplc_color_scale;
     lap *= p.w;   // 1/rho_i
     float sx = 0.f, sy = 0.f, sz = 0.f;
-    const float n2 = gx * gx + gy * gy + gz * gz;
+    const float n2 = dot3(gx, gy, gz, gx, gy, gz);
     if (sms) {
         // force_kernels.cu:1030-1043
         const float inv_n = rsqrtf(n2);
@@ -314,6 +325,20 @@ __device__ __forceinline__ void write_force(const Frame &f, const DevParams &P,
 // Cell-array bytes past which the TRA density pass prefetches its rows'
 // offsets: about half of the GB300's L2.
 constexpr size_t kRowPrefetchCellBytes = size_t(64) << 20;
+
+// Up to how many work units (32 particles) per SM the small-scene builds run:
+// k_density_tra_rows with a row per warp and with three rows per warp, and
+// the small build of k_force_tra. Frame times (CUDA graphs, 152 SMs), the
+// general builds against the small ones, us:
+//   particles (units per SM)    4,096 (0.8)  32,768 (6.7)  64,000 (13)  110,592 (23)  262,144 (54)
+//   density, a row per warp       58 / 45       65 / 54      70 / 67       80 / 87      124 / 162
+//   density, three rows           58 / 47       65 / 52      70 / 65       80 / 82      124 / 147
+//   force                         58 / 56       72 / 65      79 / 71       86 / 80      119 / 123
+// (each line with the other pass fixed). Alone, the density pass takes 7.9
+// instead of 21.2 us at 4,096 particles and the force pass 11.7 instead of 14.6.
+constexpr int kRowsMax1 = 5;
+constexpr int kRowsMax3 = 17;
+constexpr int kForceSmallMax = 27;
 
 // Warps per block of the density and force kernels: 8 by default; each
 // kernel is also built for 4 (gsph_tuning.warps_per_block), with twice the
@@ -401,6 +426,102 @@ k_density_tra(Frame f, DevParams P) {
         f.nbr_flag[idx] = incomplete ? -1 : found;
         write_density(f, P, self, sum, false);
     }
+}
+
+// The same for small scenes, with the nine rows of a work unit spread over
+// 9 / kRows warps: a lane that walks its nine rows one after the other waits
+// on some forty dependent loads, which is all the time there is when the GPU
+// holds fewer units than warps. The row warps find the masks and leave the
+// interacting candidates' h^2 - r^2 in shared memory (up to kRowTerms per
+// row); the unit's first warp then adds the terms in the order, and with the
+// operations, of k_density_tra, so both give the same bits.
+constexpr int kRowTerms = 12;
+template <int kRows>
+__global__ void __launch_bounds__(288)
+k_density_tra_rows(Frame f, DevParams P) {
+    constexpr int kWarps = 9 / kRows;       // per unit
+    constexpr int kUnits = 9 / kWarps;      // per block of 9 warps
+    __shared__ float row_term[kUnits][9][kRowTerms][32];
+    __shared__ uint32_t row_mask[kUnits][9][32];
+    __shared__ int2 row_range_sh[kUnits][9][32];
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    const int lu = warp / kWarps, part = warp % kWarps;
+    const int middle = f.ctr->middle;
+    const int u = blockIdx.x * kUnits + lu;
+    const int idx = (u << 5) + lane;
+    if (blockIdx.x * (kUnits << 5) >= middle) return;   // the whole block
+    const bool active = idx < middle;
+    const float cut = P.h2 - kFloatSmall;
+    const uint32_t cut_bits = __float_as_uint(cut);
+    int self = 0;
+    float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (active) {
+        self = f.ctr->any_sms ? f.compact[idx] : idx;
+        p = f.pos[self];
+        const SceneGeom G = geom_of_particle(f.scenes, self);
+        const MicroPos mp = micro_of(p, P, G);
+#pragma unroll
+        for (int k = 0; k < kRows; ++k) {
+            const int r = part * kRows + k;
+            const int ny = mp.cy + (r % 3) - 1;
+            const int nz = mp.cz + (r / 3) - 1;
+            uint32_t mask = 0u;
+            int begin = 0, end = 0;
+            if (ny >= 0 && ny < G.gy && nz >= 0 && nz < G.gz) {
+                row_range(f, G, G.cbase + mp.cx + G.gx * (ny + G.gy * nz), mp.cx, mp.lmx,
+                          mp.lmx, begin, end);
+                const int n = min(end - begin, kMaskRowMax);
+                int terms = 0;
+#pragma unroll 8
+                for (int j = 0; j < n; ++j) {
+                    const float4 q = f.pos[begin + j];
+                    const float e = sq_dist_less_small(p.x - q.x, p.y - q.y, p.z - q.z);
+                    if (__float_as_uint(e) > cut_bits) continue;
+                    if (terms < kRowTerms) row_term[lu][r][terms][lane] = cut - e;
+                    ++terms;
+                    mask |= 1u << j;
+                }
+            }
+            row_mask[lu][r][lane] = mask;
+            row_range_sh[lu][r][lane] = make_int2(begin, end);
+        }
+    }
+    __syncthreads();
+    if (part != 0 || !active) return;
+    uint32_t *masks = f.nbr_mask + size_t(u) * 9 * 32 + lane;
+    int found = 0;
+    bool incomplete = false;
+    float sum = 0.f;
+#pragma unroll
+    for (int r = 0; r < 9; ++r) {
+        uint32_t mask = row_mask[lu][r][lane];
+        const int2 range = row_range_sh[lu][r][lane];
+        const int n = __popc(mask);
+        masks[r * 32] = mask;
+        found += n;
+        for (int k = 0; k < min(n, kRowTerms); ++k) {
+            const float t = row_term[lu][r][k][lane];
+            sum += t * t * t;
+        }
+        auto add = [&](int j) {
+            const float4 q = f.pos[j];
+            const float e = sq_dist_less_small(p.x - q.x, p.y - q.y, p.z - q.z);
+            if (__float_as_uint(e) > cut_bits) return;
+            const float t = cut - e;
+            sum += t * t * t;
+        };
+        if (n > kRowTerms) {
+            for (int k = 0; k < kRowTerms; ++k) mask &= mask - 1u;
+            for (; mask; mask &= mask - 1u) add(range.x + __ffs(mask) - 1);
+        }
+        if (range.y - range.x > kMaskRowMax) {
+            incomplete = true;
+            for (int j = range.x + kMaskRowMax; j < range.y; ++j) add(j);
+        }
+    }
+    f.nbr_flag[idx] = incomplete ? -1 : found;
+    write_density(f, P, self, sum, false);
 }
 
 // ------------------------------------------------------- SMS candidates --
@@ -700,8 +821,14 @@ k_density_sms(Frame f, DevParams P) {
 // mask) pairs in shared memory and walks all its neighbours in one loop, so
 // lanes stay converged across rows. Without masks (or with a row longer than
 // 32 candidates) the lane scans its candidates as the reference does.
-template <bool kArt, int W>
-__global__ void __launch_bounds__(W * 32, 4 * kWarpsPerBlock / W)
+//
+// kSmall: the build for scenes with fewer work units than the GPU holds
+// warps. Each warp takes the unit of its index (no queue: thousands of idle
+// warps taking turns on one counter cost more than the work), and four
+// neighbours' loads instead of two are in flight before the first of them is
+// evaluated (the order of the sums is unchanged).
+template <bool kArt, int W, bool kSmall = false>
+__global__ void __launch_bounds__(W * 32, kSmall ? 1 : 4 * kWarpsPerBlock / W)
 k_force_tra(Frame f, DevParams P, bool fresh) {
     __shared__ uint32_t row_mask[9][W * 32];
     __shared__ int row_start[9][W * 32];
@@ -710,8 +837,10 @@ k_force_tra(Frame f, DevParams P, bool fresh) {
     const int units = (middle + 31) >> 5;
     const bool ident = !f.ctr->any_sms;   // all TRA: compact is the identity
     if (units == 0) return;        // no TRA work: skip the queue atomics
-    for (;;) {
-        const int u = next_unit(&f.ctr->work_force);
+    for (bool first = true;; first = false) {
+        if (kSmall && !first) break;
+        const int u = kSmall ? int(blockIdx.x * W + (threadIdx.x >> 5))
+                             : next_unit(&f.ctr->work_force);
         if (u >= units) break;
         const int idx = (u << 5) + lane;
         if (idx >= middle) continue;
@@ -747,9 +876,33 @@ k_force_tra(Frame f, DevParams P, bool fresh) {
             int r = 0;
             uint32_t mask = row_mask[0][threadIdx.x];
             int base = row_start[0][threadIdx.x];
-            // two neighbours per iteration: both loads are in flight before
-            // the first pair is evaluated (the order of the sums is unchanged)
+            // two (kSmall: four) neighbours per iteration: their loads are in
+            // flight before the first pair is evaluated (the order of the sums
+            // is unchanged)
             int k = 0;
+            if constexpr (kSmall) {
+                for (; k < found; k += 4) {
+                    float4 q[4], e[4];
+#pragma unroll
+                    for (int s = 0; s < 4; ++s) {
+                        int j = self;
+                        if (k + s < found) {
+                            while (!mask) {
+                                ++r;
+                                mask = row_mask[r][threadIdx.x];
+                                base = row_start[r][threadIdx.x];
+                            }
+                            j = base + __ffs(mask) - 1;
+                            mask &= mask - 1u;
+                        }
+                        q[s] = f.pos[j];
+                        e[s] = f.ev[j];
+                    }
+#pragma unroll
+                    for (int s = 0; s < 4; ++s)
+                        if (k + s < found) force_pair<false, kArt>(p, pev, q[s], e[s], P, a);
+                }
+            }
             for (; k + 1 < found; k += 2) {
                 while (!mask) {
                     ++r;
@@ -1145,7 +1298,12 @@ void launch_density_w(const Frame &f, const DevParams &P, int num_sms,
                       const LaunchShape &shape, cudaStream_t s, cudaStream_t s_sms,
                       bool row_prefetch) {
     k_density_sms<W><<<num_sms * shape.density_sms, W * 32, 0, s_sms>>>(f, P);
-    if (row_prefetch)
+    const int units = (f.n + 31) / 32;
+    if (units <= num_sms * kRowsMax1)
+        k_density_tra_rows<1><<<units, 288, 0, s>>>(f, P);
+    else if (units <= num_sms * kRowsMax3)
+        k_density_tra_rows<3><<<(units + 2) / 3, 288, 0, s>>>(f, P);
+    else if (row_prefetch)
         k_density_tra<W, true><<<num_sms * shape.density_tra, W * 32, 0, s>>>(f, P);
     else
         k_density_tra<W, false><<<num_sms * shape.density_tra, W * 32, 0, s>>>(f, P);
@@ -1155,7 +1313,11 @@ template <bool kArt, int W>
 void launch_force_w(const Frame &f, const DevParams &P, int num_sms, bool fresh,
                     const LaunchShape &shape, cudaStream_t s, cudaStream_t s_sms) {
     k_force_sms<kArt, W><<<num_sms * shape.force_sms, W * 32, 0, s_sms>>>(f, P);
-    k_force_tra<kArt, W><<<num_sms * shape.force_tra, W * 32, 0, s>>>(f, P, fresh);
+    const int units = (f.n + 31) / 32;
+    if (units <= num_sms * kForceSmallMax)
+        k_force_tra<kArt, 2, true><<<(units + 1) / 2, 64, 0, s>>>(f, P, fresh);
+    else
+        k_force_tra<kArt, W><<<num_sms * shape.force_tra, W * 32, 0, s>>>(f, P, fresh);
 }
 
 }  // namespace
