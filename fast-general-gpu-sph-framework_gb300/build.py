@@ -53,7 +53,7 @@ def build(verbose_ptxas: bool = False, force: bool = False) -> Path:
     LIB.mkdir(exist_ok=True)
     objdir = LIB / "obj"
     objdir.mkdir(exist_ok=True)
-    headers = [CSRC / "gsph_internal.h", ROOT / "include" / "gsph.h"]
+    headers = [CSRC / "gsph_internal.h", CSRC / "split_device.cuh", ROOT / "include" / "gsph.h"]
     common = ["-std=c++17", "-O3", "-Xcompiler", "-fPIC", f"-I{ROOT / 'include'}"]
     jobs = []
     for src in CUDA_SOURCES:

@@ -14,8 +14,12 @@
 //   * counting is per COARSE cell (numc ints, not numc*64), with warp-aggregated
 //     atomics (match.any) so a warp of sorted particles issues one atomic per
 //     cell it touches;
-//   * the coarse scan is reduce-then-scan (no inter-CTA spin waits) and also
-//     compacts the occupied cells and the list of large cells;
+//   * the coarse scan is reduce-then-scan (no inter-CTA waits), a single pass
+//     for small grids; it also compacts the occupied cells and the list of
+//     large cells;
+//   * the performance model and the TRA/SMS split run inside the sort's own
+//     launches, where the data they need is ready, so that the arrange stage
+//     is four launches (five for large grids);
 //   * the order inside a coarse cell is canonical: (micro key, previous index).
 //     The reference's atomic slot order varies run to run; this one does not,
 //     so two runs (and the CPU restatement) give the same permutation;
@@ -24,7 +28,7 @@
 //     because every use clamps them by the cell's count.
 #include <algorithm>
 
-#include "gsph_internal.h"
+#include "split_device.cuh"
 
 namespace gsph {
 
@@ -76,9 +80,8 @@ k_hash_sms(const float4 *__restrict__ pos, int n, DevParams P, SceneTable T,
 }
 
 // ---------------------------------------------------------------------------
-// A3/A5: reduce-then-scan over the coarse counts. Values are packed
-// (occupied << 32) | count so one scan yields the cell offsets and the
-// occupied-cell compaction.
+// A3/A5: scan over the coarse counts. Values are packed (occupied << 32) |
+// count so one scan yields the cell offsets and the occupied-cell compaction.
 __device__ __forceinline__ unsigned long long pack_cell(int cnt) {
     return (cnt > 0 ? (1ull << 32) : 0ull) | (unsigned long long)(unsigned)cnt;
 }
@@ -103,116 +106,76 @@ __device__ __forceinline__ void load_tile_counts(const int32_t *__restrict__ in,
     }
 }
 
-// Exclusive scan of the packed tile sums by one block (any multiple of 32
-// threads), in place; returns the grand total to thread 0. The tiles were
-// written by other CTAs of the same launch, so they are read from L2.
-__device__ unsigned long long scan_tile_sums(unsigned long long *tiles, int ntiles) {
-    __shared__ unsigned long long ws[32];
-    __shared__ unsigned long long carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nw = int(blockDim.x >> 5);
-    for (int base = 0; base < ntiles; base += blockDim.x) {
-        const int t = base + threadIdx.x;
-        const unsigned long long v = t < ntiles ? __ldcg(tiles + t) : 0ull;
-        unsigned long long x = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            unsigned long long y = __shfl_up_sync(kFull, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) ws[warp] = x;
-        __syncthreads();
-        if (warp == 0) {
-            unsigned long long w = lane < nw ? ws[lane] : 0ull;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                unsigned long long y = __shfl_up_sync(kFull, w, o);
-                if (lane >= o) w += y;
-            }
-            if (lane < nw) ws[lane] = w;
-        }
-        __syncthreads();
-        const unsigned long long wprefix = warp > 0 ? ws[warp - 1] : 0ull;
-        const unsigned long long excl = carry + wprefix + x - v;
-        if (t < ntiles) tiles[t] = excl;
-        __syncthreads();
-        if (threadIdx.x == blockDim.x - 1) carry = excl + v;
-        __syncthreads();
-    }
-    return carry;
-}
-
-// Tile sums of the packed (occupied, count) values; the last CTA to finish
-// (a counter, no waiting) scans the tile sums, writes the grand total and
-// resets the frame's work counters.
+// Sum of every tile of kScanTile cells.
 __global__ void __launch_bounds__(kScanThreads)
-k_cell_scan_reduce(const int32_t *__restrict__ count, int numc,
-                   unsigned long long *__restrict__ tiles, int32_t *__restrict__ cell_start,
-                   Counters *ctr) {
-    const int first = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
+k_tile_sums(const int32_t *__restrict__ count, int numc,
+            unsigned long long *__restrict__ tiles) {
     int v[kScanItems];
-    load_tile_counts(count, numc, first, v);
+    load_tile_counts(count, numc, blockIdx.x * kScanTile + threadIdx.x * kScanItems, v);
     unsigned long long s = 0;
 #pragma unroll
     for (int q = 0; q < kScanItems; ++q) s += pack_cell(v[q]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(kFull, s, o);
     __shared__ unsigned long long ws[kScanThreads / 32];
-    __shared__ bool last;
     if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned long long t = 0;
         for (int w = 0; w < kScanThreads / 32; ++w) t += ws[w];
         tiles[blockIdx.x] = t;
-        __threadfence();
-        last = atomicAdd(&ctr->scan_done, 1) == int(gridDim.x) - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    const unsigned long long total = scan_tile_sums(tiles, int(gridDim.x));
-    if (threadIdx.x == 0) {
-        cell_start[numc] = int32_t(total & 0xFFFFFFFFull);
-        ctr->num_occ = int32_t(total >> 32);
-        ctr->num_big = 0;
-        ctr->work_density = 0;
-        ctr->work_force = 0;
-        ctr->work_density_sms = 0;
-        ctr->work_force_sms = 0;
-        ctr->any_sms = 0;
-        ctr->scan_done = 0;
     }
 }
 
+// The scan, one tile per CTA; a CTA adds up what lies before its tile itself:
+// the sums of the earlier tiles (at most 16,384 of them, read from L2) or, in
+// the direct build, their counts, which for up to kScanDirectTiles tiles takes
+// less time than the launch of k_tile_sums (frame of 13,824 particles, 4 tiles,
+// 39.1 against 40.2 us; of 46,656, 13 tiles, 58.3 against 55.9). (Tile sums kept by the hash's
+// atomics instead need no pass at all, but contend: hash 24 -> 236 us for
+// 3.94M particles in 38 tiles.) The last tile's CTA writes the grand total and
+// resets the frame's counters.
+template <bool kDirect>
 __global__ void __launch_bounds__(kScanThreads)
-k_cell_scan_apply(const int32_t *__restrict__ count, int numc,
-                  const unsigned long long *__restrict__ tiles,
-                  int32_t *__restrict__ cell_start,
-                  int32_t *__restrict__ occ_list,
-                  int32_t *__restrict__ big_list, Counters *ctr) {
+k_cell_scan(const int32_t *__restrict__ count, int numc,
+            const unsigned long long *__restrict__ tiles,
+            int32_t *__restrict__ cell_start, int32_t *__restrict__ occ_list,
+            int32_t *__restrict__ big_list, Counters *ctr, int n_particles) {
     const int first = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     int v[kScanItems];
     load_tile_counts(count, numc, first, v);
     unsigned long long s = 0;
 #pragma unroll
     for (int q = 0; q < kScanItems; ++q) s += pack_cell(v[q]);
-    // block exclusive scan of per-thread sums
+    unsigned long long before = 0;
+    if (kDirect) {
+        const int4 *c4 = reinterpret_cast<const int4 *>(count);
+        int cnt = 0, occ = 0;
+#pragma unroll 8
+        for (int t = threadIdx.x; t < int(blockIdx.x) * (kScanTile / 4); t += kScanThreads) {
+            const int4 c = c4[t];
+            cnt += c.x + c.y + c.z + c.w;
+            occ += min(c.x, 1) + min(c.y, 1) + min(c.z, 1) + min(c.w, 1);
+        }
+        before = ((unsigned long long)(unsigned)occ << 32) | (unsigned)cnt;
+    } else {
+        for (int t = threadIdx.x; t < int(blockIdx.x); t += kScanThreads) before += tiles[t];
+    }
+    // block exclusive scan of per-thread sums, and the sum of `before`
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned long long x = s;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         unsigned long long y = __shfl_up_sync(kFull, x, o);
         if (lane >= o) x += y;
+        before += __shfl_xor_sync(kFull, before, o);
     }
-    __shared__ unsigned long long ws[kScanThreads / 32];
+    __shared__ unsigned long long ws[kScanThreads / 32], wb[kScanThreads / 32];
     if (lane == 31) ws[warp] = x;
+    if (lane == 0) wb[warp] = before;
     __syncthreads();
-    unsigned long long wprefix = 0;
-    for (int w = 0; w < warp; ++w) wprefix += ws[w];
-    unsigned long long run = tiles[blockIdx.x] + wprefix + x - s;
+    unsigned long long run = x - s;
+    for (int w = 0; w < kScanThreads / 32; ++w) run += wb[w] + (w < warp ? ws[w] : 0ull);
     int out[kScanItems];
 #pragma unroll
     for (int q = 0; q < kScanItems; ++q) {
@@ -220,7 +183,8 @@ k_cell_scan_apply(const int32_t *__restrict__ count, int numc,
         out[q] = int32_t(run & 0xFFFFFFFFull);
         if (c < numc && v[q] > 0) {
             occ_list[run >> 32] = c;
-            if (v[q] > kSmallCellMax) big_list[atomicAdd(&ctr->num_big, 1)] = c;
+            if (v[q] > kSmallCellMax)
+                big_list[atomicAdd(&ctr->big_fill, 1)] = int32_t(run >> 32);
         }
         run += pack_cell(v[q]);
     }
@@ -235,19 +199,49 @@ k_cell_scan_apply(const int32_t *__restrict__ count, int numc,
         for (int q = 0; q < kScanItems; ++q)
             if (first + q < numc) cell_start[first + q] = out[q];
     }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == kScanThreads - 1) {
+        cell_start[numc] = int32_t(run & 0xFFFFFFFFull);
+        ctr->num_occ = int32_t(run >> 32);
+        ctr->work_density = 0;
+        ctr->work_force = 0;
+        ctr->work_density_sms = 0;
+        ctr->work_force_sms = 0;
+        // all TRA, unless the performance model finds an SMS cell
+        ctr->any_sms = 0;
+        ctr->task_count = 0;
+        ctr->n_sms = 0;
+        ctr->middle = n_particles;
+    }
 }
 
 // ---------------------------------------------------------------------------
-// Scatter (key, source) pairs to their coarse-cell range (slot order).
-__global__ void __launch_bounds__(256)
-k_scatter_pairs(const uint32_t *__restrict__ key_in,
-                const uint32_t *__restrict__ slot, int n,
-                const int32_t *__restrict__ cell_start,
-                unsigned long long *__restrict__ pairs) {
+// Scatter (key, source) pairs to their coarse-cell range (slot order), after
+// `model_blocks` blocks of the performance model, which like the scatter
+// needs nothing but the cell offsets: in small scenes the two overlap (4,096
+// particles 5.2 us against 2.9 + 5.5 as two launches; 3.94M 23.7 against 12.6
+// + 10.3). Also publishes the number of large cells.
+__global__ void __launch_bounds__(kScanThreads)
+k_scatter(Frame f, DevParams P, int model_blocks) {
+    if (int(blockIdx.x) < model_blocks) {
+        const int num_occ = f.ctr->num_occ;
+        for (int tile = blockIdx.x; tile * kValTile < num_occ; tile += model_blocks)
+            model_tile(f, P, tile, num_occ);
+        return;
+    }
+    const int block = blockIdx.x - model_blocks;
+    const int n = f.n;
+    const uint32_t *__restrict__ key_in = f.key_in;
+    const uint32_t *__restrict__ slot = f.slot;
+    const int32_t *__restrict__ cell_start = f.cell_start;
+    unsigned long long *__restrict__ pairs = f.pairs;
+    if (block == 0 && threadIdx.x == 0) {
+        f.ctr->num_big = f.ctr->big_fill;
+        f.ctr->big_fill = 0;
+    }
     // two particles per thread, a block-width apart: both chains of loads
     // are in flight together
-    const int i0 = blockIdx.x * (2 * blockDim.x) + threadIdx.x;
-    const int i1 = i0 + blockDim.x;
+    const int i0 = block * (2 * kScanThreads) + threadIdx.x;
+    const int i1 = i0 + kScanThreads;
     uint32_t k0 = 0, k1 = 0, s0 = 0, s1 = 0;
     if (i0 < n) { k0 = key_in[i0]; s0 = slot[i0]; }
     if (i1 < n) { k1 = key_in[i1]; s1 = slot[i1]; }
@@ -321,9 +315,16 @@ __device__ __forceinline__ void small_cell_groups(const Frame &f, uint32_t cell,
 // thread takes two particles a block-width apart and issues both particles'
 // loads (pair, cell bounds, state, the cell's pairs) before any store, so
 // that the two chains of loads are in flight together.
+// Where a split is made, the first block scans the performance model's tile
+// sums instead.
 __global__ void __launch_bounds__(256) k_sort_small(Frame f) {
+    int block = blockIdx.x;
+    if (f.cell_val && block-- == 0) {
+        model_totals(f);
+        return;
+    }
     int s[2];
-    s[0] = blockIdx.x * (2 * blockDim.x) + threadIdx.x;
+    s[0] = block * (2 * blockDim.x) + threadIdx.x;
     s[1] = s[0] + blockDim.x;
     unsigned long long e[2] = {0ull, 0ull};
     int b[2] = {0, 0}, cnt[2] = {0, 0}, rank[2] = {0, 0};
@@ -418,17 +419,30 @@ __device__ void block_exclusive_scan(const int *in, int *out, int n) {
 // compare as (micro cell, source index) inside a cell, so up to kBigCellSmem
 // particles the pairs are staged in shared memory, bucketed by their 6-bit
 // micro cell (counts, scan, scatter) and ranked by value inside their bucket
-// only. Larger cells do the same in global memory with finer buckets.
+// only. Larger cells do the same in global memory with finer buckets. In a
+// frame with SMS cells the block then emits its cell's part of the compact
+// index and its tasks, and the cells of k_sort_small are emitted one per
+// thread (default scene, 3.94M particles: arrange 332 -> 290 us; with a thread
+// writing all of a 280-particle cell the emission alone took 41 us, and 34 of
+// 64,000 particles' 88).
 __global__ void __launch_bounds__(256) k_sort_big(Frame f) {
     __shared__ unsigned long long sp[kBigCellSmem];
     __shared__ uint16_t order[kBigCellSmem];
     __shared__ int mcount[64], mfill[64], mstart[65];
     __shared__ int grp[16];
     const int nbig = f.ctr->num_big;
+    const bool emit = f.cell_val && f.ctr->any_sms;
     for (int q = blockIdx.x; q < nbig; q += gridDim.x) {
-        const int cell = f.big_list[q];
+        const int place = f.big_list[q];
+        const int cell = f.occ_list[place];
         const int b = f.cell_start[cell];
         const int cnt = f.cell_start[cell + 1] - b;
+        // loaded here, so that they are there when the cell is sorted
+        int4 val = make_int4(0, 0, 0, 0), before = val;
+        if (emit) {
+            val = f.cell_val[place];
+            before = cells_before(f, place);
+        }
         if (cnt <= kBigCellSmem) {
             if (threadIdx.x < 64) {
                 mcount[threadIdx.x] = 0;
@@ -476,6 +490,14 @@ __global__ void __launch_bounds__(256) k_sort_big(Frame f) {
                 write_groups(f, uint32_t(cell), n16, cnt);
                 f.cell_count[cell] = 0;
             }
+            if (emit)
+                emit_cell(f, cell, b, cnt, val, before, threadIdx.x, blockDim.x, [&](int i) {
+                    int lo = 0;   // the micro cell m with mstart[m] <= i < mstart[m + 1]
+#pragma unroll
+                    for (int s = 32; s > 0; s >>= 1)
+                        if (mstart[lo + s] <= i) lo += s;
+                    return uint32_t(lo);
+                });
             __syncthreads();
             continue;
         }
@@ -528,6 +550,20 @@ __global__ void __launch_bounds__(256) k_sort_big(Frame f) {
             f.cell_count[cell] = 0;
         }
         __syncthreads();
+        if (emit)
+            emit_cell(f, cell, b, cnt, val, before, threadIdx.x, blockDim.x,
+                      [&](int i) { return f.key[b + i]; });
+    }
+    if (!emit) return;   // all TRA: the compact index is the identity
+    const int num_occ = f.ctr->num_occ;
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < num_occ;
+         k += gridDim.x * blockDim.x) {
+        const int cell = f.occ_list[k];
+        const int b = f.cell_start[cell];
+        const int n = f.cell_start[cell + 1] - b;
+        if (n <= kSmallCellMax)
+            emit_cell(f, cell, b, n, f.cell_val[k], cells_before(f, k), 0, 1,
+                      [&](int i) { return f.key[b + i]; });
     }
 }
 
@@ -549,22 +585,33 @@ void launch_hash_count(const Frame &f, const DevParams &P, cudaStream_t s) {
 
 void launch_cell_scan(const Frame &f, const DevParams &P, cudaStream_t s) {
     const int ntiles = (P.numc + kScanTile - 1) / kScanTile;
-    k_cell_scan_reduce<<<ntiles, kScanThreads, 0, s>>>(f.cell_count, P.numc,
-                                                       f.scan_tiles, f.cell_start, f.ctr);
-    k_cell_scan_apply<<<ntiles, kScanThreads, 0, s>>>(
-        f.cell_count, P.numc, f.scan_tiles, f.cell_start, f.occ_list,
-        f.big_list, f.ctr);
+    if (ntiles <= kScanDirectTiles) {
+        k_cell_scan<true><<<ntiles, kScanThreads, 0, s>>>(f.cell_count, P.numc, nullptr,
+                                                          f.cell_start, f.occ_list,
+                                                          f.big_list, f.ctr, f.n);
+        return;
+    }
+    k_tile_sums<<<ntiles, kScanThreads, 0, s>>>(f.cell_count, P.numc, f.scan_tiles);
+    k_cell_scan<false><<<ntiles, kScanThreads, 0, s>>>(f.cell_count, P.numc, f.scan_tiles,
+                                                       f.cell_start, f.occ_list, f.big_list,
+                                                       f.ctr, f.n);
 }
 
-void launch_scatter_pairs(const Frame &f, cudaStream_t s) {
+void launch_scatter(const Frame &f, const DevParams &P, int max_occ, int num_sms,
+                    cudaStream_t s) {
     if (f.n <= 0) return;
-    k_scatter_pairs<<<(f.n + 511) / 512, 256, 0, s>>>(f.key_in, f.slot, f.n,
-                                                     f.cell_start, f.pairs);
+    // grid-stride over the device-side count, sized for the capacity but at
+    // most a few blocks per SM
+    const int model = f.cell_val
+                          ? std::min((max_occ + kValTile - 1) / kValTile, num_sms * 8)
+                          : 0;
+    k_scatter<<<model + (f.n + 2 * kScanThreads - 1) / (2 * kScanThreads), kScanThreads, 0,
+                s>>>(f, P, model);
 }
 
 void launch_cell_sort(const Frame &f, int num_sms, cudaStream_t s) {
     if (f.n <= 0) return;
-    k_sort_small<<<(f.n + 511) / 512, 256, 0, s>>>(f);
+    k_sort_small<<<(f.n + 511) / 512 + (f.cell_val ? 1 : 0), 256, 0, s>>>(f);
     k_sort_big<<<num_sms * 4, 256, 0, s>>>(f);
 }
 

@@ -42,6 +42,8 @@ constexpr int kMaskRowMax = 32;
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 16;
 constexpr int kScanTile = kScanThreads * kScanItems;
+// Up to this many tiles the cell scan needs no tile sums (k_cell_scan).
+constexpr int kScanDirectTiles = 6;
 // Tiles of the per-occupied-cell {tasks, SMS, TRA} scan of the split.
 constexpr int kValItems = 4;
 constexpr int kValTile = kScanThreads * kValItems;
@@ -135,11 +137,8 @@ struct Counters {
     // particle is TRA, the compact index is the identity and the TRA/SMS
     // compaction is skipped.
     int32_t any_sms;
-    // CTAs of the cell-count reduction / of the performance model that have
-    // written their tile sums; the last one scans the tiles (and resets it).
-    int32_t scan_done;
-    int32_t model_done;
-    int32_t pad[18];
+    int32_t big_fill;       // large cells listed so far by the cell scan
+    int32_t pad[19];
 };
 
 // Per-frame device pointers of one batch of scenes.
@@ -168,9 +167,11 @@ struct Frame {
     // entry 0 is kGroupsUnknown for cells above 65,535 particles. Null when the
     // caller does not keep it.
     uint16_t *cell_grp;
-    int32_t *occ_list, *big_list;
-    int4 *cell_val;                            // per occupied cell {req,sms,tra}
-    int4 *cell_prefix;                         // exclusive prefix of cell_val
+    int32_t *occ_list;                         // occupied cells, in order
+    int32_t *big_list;                         // large cells' places in occ_list
+    int4 *cell_val;                            // per occupied cell {req,sms,tra};
+                                               // null: sort only, no split
+    int4 *cell_prefix;                         // exclusive prefix inside its tile
     gsph_block_task *tasks;
     int32_t task_capacity;
     int32_t *compact;
@@ -247,19 +248,19 @@ __device__ __forceinline__ uint32_t cell_slot(int32_t *cell_count, uint32_t cell
 
 // ---- launchers (grid.cu) ----
 void launch_hash_count(const Frame &f, const DevParams &P, cudaStream_t s);
-// Hash of the previous split's SMS particles only (compact[middle, n)).
 // Keys and cell slots ahead for the split's SMS particles (compact[middle,
 // n)) from their integrated positions `pos`.
 void launch_hash_sms(const Frame &f, const float4 *pos, const DevParams &P,
                      cudaStream_t s);
 void launch_cell_scan(const Frame &f, const DevParams &P, cudaStream_t s);
-void launch_scatter_pairs(const Frame &f, cudaStream_t s);
+// The pair scatter and, where f.cell_val is set, the performance model of the
+// occupied cells (at most max_occ).
+void launch_scatter(const Frame &f, const DevParams &P, int max_occ, int num_sms,
+                    cudaStream_t s);
+// The order inside the cells and, where f.cell_val is set, the TRA/SMS
+// partition and the SMS tasks; launch_judge then pairs the tasks (judgeTask).
 void launch_cell_sort(const Frame &f, int num_sms, cudaStream_t s);
 // ---- launchers (split.cu) ----
-// Performance model, TRA/SMS partition and SMS tasks; launch_judge then
-// pairs the tasks (judgeTask), which only the SMS passes read.
-void launch_split(const Frame &f, const DevParams &P, int max_occ, int num_sms,
-                  cudaStream_t s);
 void launch_judge(const Frame &f, int max_occ, int num_sms, cudaStream_t s);
 // ---- launchers (physics.cu) ----
 // Launch shapes of the density and force passes: CTAs per SM of each kernel.

@@ -535,9 +535,8 @@ struct System {
         const Frame f = frame_arrange(in);
         if (!hashed) enqueue_hash(in);
         launch_cell_scan(f, dp, stream);
-        launch_scatter_pairs(f, stream);
+        launch_scatter(f, dp, max_occ, num_sms, stream);
         launch_cell_sort(f, num_sms, stream);
-        launch_split(f, dp, max_occ, num_sms, stream);
         if (pair_tasks) launch_judge(f, max_occ, num_sms, stream);
         hashed = false;          // consumed; the sort cleared the counts
         counts_dirty = false;
@@ -1956,18 +1955,20 @@ gsph_status gsph_grid_sort_dev(const gsph_params *p, uint32_t n,
     f.key_in = reinterpret_cast<uint32_t *>(carve(N * 4));
     f.slot = reinterpret_cast<uint32_t *>(carve(N * 4));
     f.pairs = reinterpret_cast<unsigned long long *>(carve(N * 8));
-    f.cell_count = reinterpret_cast<int32_t *>(carve(C * 4));
     f.cell_xslab = reinterpret_cast<uint32_t *>(carve(C * 4));
     f.occ_list = reinterpret_cast<int32_t *>(carve(occ * 4));
     f.big_list = reinterpret_cast<int32_t *>(carve(occ * 4));
-    f.scan_tiles = reinterpret_cast<unsigned long long *>(carve(tiles * 8));
+    // what the sort accumulates into, side by side: cleared by one memset
+    char *const sums = w;
+    f.cell_count = reinterpret_cast<int32_t *>(carve(C * 4));
     f.ctr = reinterpret_cast<Counters *>(carve(sizeof(Counters)));
+    const size_t sum_bytes = size_t(w - sums);
+    f.scan_tiles = reinterpret_cast<unsigned long long *>(carve(tiles * 8));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    GSPH_CUDA(cudaMemsetAsync(f.cell_count, 0, C * 4, s));
-    GSPH_CUDA(cudaMemsetAsync(f.ctr, 0, sizeof(Counters), s));
+    GSPH_CUDA(cudaMemsetAsync(sums, 0, sum_bytes, s));
     launch_hash_count(f, dp, s);
     launch_cell_scan(f, dp, s);
-    launch_scatter_pairs(f, s);
+    launch_scatter(f, dp, int(occ), device_sm_count(dev), s);
     launch_cell_sort(f, device_sm_count(dev), s);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
