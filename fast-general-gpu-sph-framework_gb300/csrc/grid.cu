@@ -110,6 +110,7 @@ __device__ __forceinline__ void load_tile_counts(const int32_t *__restrict__ in,
 __global__ void __launch_bounds__(kScanThreads)
 k_tile_sums(const int32_t *__restrict__ count, int numc,
             unsigned long long *__restrict__ tiles) {
+    chain_next();
     int v[kScanItems];
     load_tile_counts(count, numc, blockIdx.x * kScanTile + threadIdx.x * kScanItems, v);
     unsigned long long s = 0;
@@ -141,6 +142,8 @@ k_cell_scan(const int32_t *__restrict__ count, int numc,
             const unsigned long long *__restrict__ tiles,
             int32_t *__restrict__ cell_start, int32_t *__restrict__ occ_list,
             int32_t *__restrict__ big_list, Counters *ctr, int n_particles) {
+    chain_wait();
+    chain_next();
     const int first = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     int v[kScanItems];
     load_tile_counts(count, numc, first, v);
@@ -222,6 +225,8 @@ k_cell_scan(const int32_t *__restrict__ count, int numc,
 // + 10.3). Also publishes the number of large cells.
 __global__ void __launch_bounds__(kScanThreads)
 k_scatter(Frame f, DevParams P, int model_blocks) {
+    chain_wait();
+    chain_next();
     if (int(blockIdx.x) < model_blocks) {
         const int num_occ = f.ctr->num_occ;
         for (int tile = blockIdx.x; tile * kValTile < num_occ; tile += model_blocks)
@@ -318,6 +323,8 @@ __device__ __forceinline__ void small_cell_groups(const Frame &f, uint32_t cell,
 // Where a split is made, the first block scans the performance model's tile
 // sums instead.
 __global__ void __launch_bounds__(256) k_sort_small(Frame f) {
+    chain_wait();
+    chain_next();
     int block = blockIdx.x;
     if (f.cell_val && block-- == 0) {
         model_totals(f);
@@ -430,6 +437,8 @@ __global__ void __launch_bounds__(256) k_sort_big(Frame f) {
     __shared__ uint16_t order[kBigCellSmem];
     __shared__ int mcount[64], mfill[64], mstart[65];
     __shared__ int grp[16];
+    chain_wait();
+    chain_next();
     const int nbig = f.ctr->num_big;
     const bool emit = f.cell_val && f.ctr->any_sms;
     for (int q = blockIdx.x; q < nbig; q += gridDim.x) {
@@ -592,9 +601,8 @@ void launch_cell_scan(const Frame &f, const DevParams &P, cudaStream_t s) {
         return;
     }
     k_tile_sums<<<ntiles, kScanThreads, 0, s>>>(f.cell_count, P.numc, f.scan_tiles);
-    k_cell_scan<false><<<ntiles, kScanThreads, 0, s>>>(f.cell_count, P.numc, f.scan_tiles,
-                                                       f.cell_start, f.occ_list, f.big_list,
-                                                       f.ctr, f.n);
+    launch_after(k_cell_scan<false>, ntiles, kScanThreads, s, f.cell_count, P.numc,
+                 f.scan_tiles, f.cell_start, f.occ_list, f.big_list, f.ctr, f.n);
 }
 
 void launch_scatter(const Frame &f, const DevParams &P, int max_occ, int num_sms,
@@ -605,14 +613,14 @@ void launch_scatter(const Frame &f, const DevParams &P, int max_occ, int num_sms
     const int model = f.cell_val
                           ? std::min((max_occ + kValTile - 1) / kValTile, num_sms * 8)
                           : 0;
-    k_scatter<<<model + (f.n + 2 * kScanThreads - 1) / (2 * kScanThreads), kScanThreads, 0,
-                s>>>(f, P, model);
+    launch_after(k_scatter, model + (f.n + 2 * kScanThreads - 1) / (2 * kScanThreads),
+                 kScanThreads, s, f, P, model);
 }
 
 void launch_cell_sort(const Frame &f, int num_sms, cudaStream_t s) {
     if (f.n <= 0) return;
-    k_sort_small<<<(f.n + 511) / 512 + (f.cell_val ? 1 : 0), 256, 0, s>>>(f);
-    k_sort_big<<<num_sms * 4, 256, 0, s>>>(f);
+    launch_after(k_sort_small, (f.n + 511) / 512 + (f.cell_val ? 1 : 0), 256, s, f);
+    launch_after(k_sort_big, num_sms * 4, 256, s, f);
 }
 
 }  // namespace gsph

@@ -197,6 +197,34 @@ inline __host__ __device__ void set_task_offset(gsph_block_task &t, int off) {
 }
 
 #ifdef __CUDACC__
+// Programmatic dependent launch: a kernel launched by launch_after may be
+// scheduled while the kernel before it in its stream still runs; chain_wait,
+// the first statement of every such kernel, holds each thread until that
+// kernel's grid has completed and its writes are visible, and chain_next lets
+// the kernel after it be scheduled. Both do nothing in ordinary launches. It
+// takes the launch latency out of the short kernels that follow one another
+// in a frame.
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void chain_next() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... Params, class... Args>
+inline void launch_after(void (*kernel)(Params...), int grid, int block, cudaStream_t s,
+                         Args... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(grid));
+    cfg.blockDim = dim3(unsigned(block));
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, Params(args)...);   // errors: cudaGetLastError
+}
+
 __device__ __forceinline__ unsigned lanemask_lt() {
     unsigned m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));

@@ -367,6 +367,7 @@ __device__ __forceinline__ int next_unit(int *counter) {
 template <int W, bool kRowPrefetch>
 __global__ void __launch_bounds__(W * 32, 6 * kWarpsPerBlock / W)
 k_density_tra(Frame f, DevParams P) {
+    chain_wait();
     const int lane = threadIdx.x & 31;
     const int middle = f.ctr->middle;
     const int units = (middle + 31) >> 5;
@@ -437,8 +438,9 @@ k_density_tra(Frame f, DevParams P) {
 // operations, of k_density_tra, so both give the same bits.
 constexpr int kRowTerms = 12;
 template <int kRows>
-__global__ void __launch_bounds__(288)
+__global__ void __launch_bounds__(288, kRows == 1 ? 5 : 3)
 k_density_tra_rows(Frame f, DevParams P) {
+    chain_wait();
     constexpr int kWarps = 9 / kRows;       // per unit
     constexpr int kUnits = 9 / kWarps;      // per block of 9 warps
     __shared__ float row_term[kUnits][9][kRowTerms][32];
@@ -1300,13 +1302,13 @@ void launch_density_w(const Frame &f, const DevParams &P, int num_sms,
     k_density_sms<W><<<num_sms * shape.density_sms, W * 32, 0, s_sms>>>(f, P);
     const int units = (f.n + 31) / 32;
     if (units <= num_sms * kRowsMax1)
-        k_density_tra_rows<1><<<units, 288, 0, s>>>(f, P);
+        launch_after(k_density_tra_rows<1>, units, 288, s, f, P);
     else if (units <= num_sms * kRowsMax3)
-        k_density_tra_rows<3><<<(units + 2) / 3, 288, 0, s>>>(f, P);
+        launch_after(k_density_tra_rows<3>, (units + 2) / 3, 288, s, f, P);
     else if (row_prefetch)
-        k_density_tra<W, true><<<num_sms * shape.density_tra, W * 32, 0, s>>>(f, P);
+        launch_after(k_density_tra<W, true>, num_sms * shape.density_tra, W * 32, s, f, P);
     else
-        k_density_tra<W, false><<<num_sms * shape.density_tra, W * 32, 0, s>>>(f, P);
+        launch_after(k_density_tra<W, false>, num_sms * shape.density_tra, W * 32, s, f, P);
 }
 
 template <bool kArt, int W>
