@@ -144,47 +144,72 @@ __device__ __forceinline__ float artificial_pair(float vr, float d2, float k,
     return pij * k * k * inv_d;
 }
 
+// What one interacting pair adds to the accumulator: pressure -r ps, viscosity
+// u wk, gradient r gw, laplacian wh lf. kArt: the viscosity slots hold
+// Monaghan's sum_j Pi (h - r)^2 / r r_ij instead of the reference's Laplacian
+// term.
+struct PairTerms {
+    float rx, ry, rz, ps;
+    float ux, uy, uz, wk;
+    float gw, wh, lf;
+};
+template <bool kArt>
+__device__ __forceinline__ PairTerms pair_terms(const float4 &self, const float4 &sev,
+                                                const float4 &q, const float4 &qev,
+                                                const DevParams &P) {
+    PairTerms t;
+    t.rx = self.x - q.x;
+    t.ry = self.y - q.y;
+    t.rz = self.z - q.z;
+    const float d2 = sq_dist(t.rx, t.ry, t.rz);
+    const float inv_d = rsqrtf(d2);
+    const float k = __fmaf_rn(-d2, inv_d, P.h);   // h - r
+    const float V = q.w;                          // 1/rho_j
+    const float wk = V * k;
+    t.ps = wk * (sev.w + qev.w) * k * inv_d;
+    if (kArt) {
+        const float vr =
+            dot3(sev.x - qev.x, sev.y - qev.y, sev.z - qev.z, t.rx, t.ry, t.rz);
+        t.ux = t.rx;
+        t.uy = t.ry;
+        t.uz = t.rz;
+        t.wk = artificial_pair(vr, d2, k, inv_d, self.w, V, P);
+    } else {
+        t.ux = qev.x - sev.x;
+        t.uy = qev.y - sev.y;
+        t.uz = qev.z - sev.z;
+        t.wk = wk;
+    }
+    const float h2r2 = P.h2 - d2;
+    t.wh = V * h2r2;
+    t.gw = t.wh * h2r2;
+    t.lf = __fmaf_rn(-0.75f, h2r2, d2);
+    return t;
+}
+
 // kChecked = false for neighbours taken from the density pass's masks: the
 // masks were set by the same squared distance and the same cut-off test, so
-// the test would always pass. kArt: the viscosity slots of the accumulator
-// hold Monaghan's sum_j Pi (h - r)^2 / r r_ij instead of the reference's
-// Laplacian term.
+// the test would always pass.
 template <bool kChecked = true, bool kArt = false>
 __device__ __forceinline__ void force_pair(const float4 &self,
                                            const float4 &sev, const float4 &q,
                                            const float4 &qev,
                                            const DevParams &P, ForceAcc &a) {
-    const float rx = self.x - q.x, ry = self.y - q.y, rz = self.z - q.z;
-    const float d2 = sq_dist(rx, ry, rz);
-    if (kChecked && (P.h2 < d2 || kFloatSmall > d2)) return;
-    const float inv_d = rsqrtf(d2);
-    const float d = d2 * inv_d;
-    const float V = q.w;   // 1/rho_j
-    const float k = P.h - d;
-    const float wk = V * k;
-    const float pw = wk * (sev.w + qev.w) * k;
-    const float ps = pw * inv_d;
-    a.px -= rx * ps;
-    a.py -= ry * ps;
-    a.pz -= rz * ps;
-    if (kArt) {
-        const float vr = dot3(sev.x - qev.x, sev.y - qev.y, sev.z - qev.z, rx, ry, rz);
-        const float w = artificial_pair(vr, d2, k, inv_d, self.w, V, P);
-        a.vx += rx * w;
-        a.vy += ry * w;
-        a.vz += rz * w;
-    } else {
-        a.vx += (qev.x - sev.x) * wk;
-        a.vy += (qev.y - sev.y) * wk;
-        a.vz += (qev.z - sev.z) * wk;
+    if (kChecked) {
+        const float d2 = sq_dist(self.x - q.x, self.y - q.y, self.z - q.z);
+        if (P.h2 < d2 || kFloatSmall > d2) return;
     }
-    const float h2r2 = P.h2 - d2;
-    const float wh = V * h2r2;
-    const float gw = wh * h2r2;
-    a.gx += rx * gw;
-    a.gy += ry * gw;
-    a.gz += rz * gw;
-    a.lap += wh * (d2 - 0.75f * h2r2);
+    const PairTerms t = pair_terms<kArt>(self, sev, q, qev, P);
+    a.px = __fmaf_rn(t.rx, -t.ps, a.px);
+    a.py = __fmaf_rn(t.ry, -t.ps, a.py);
+    a.pz = __fmaf_rn(t.rz, -t.ps, a.pz);
+    a.vx = __fmaf_rn(t.ux, t.wk, a.vx);
+    a.vy = __fmaf_rn(t.uy, t.wk, a.vy);
+    a.vz = __fmaf_rn(t.uz, t.wk, a.vz);
+    a.gx = __fmaf_rn(t.rx, t.gw, a.gx);
+    a.gy = __fmaf_rn(t.ry, t.gw, a.gy);
+    a.gz = __fmaf_rn(t.rz, t.gw, a.gz);
+    a.lap = __fmaf_rn(t.wh, t.lf, a.lap);
 }
 
 __device__ __forceinline__ void write_density(const Frame &f, const DevParams &P,
@@ -334,10 +359,14 @@ constexpr size_t kRowPrefetchCellBytes = size_t(64) << 20;
 //   density, a row per warp       58 / 45       65 / 54      70 / 67       80 / 87      124 / 162
 //   density, three rows           58 / 47       65 / 52      70 / 65       80 / 82      124 / 147
 //   force                         58 / 56       72 / 65      79 / 71       86 / 80      119 / 123
-// (each line with the other pass fixed). Alone, the density pass takes 7.9
-// instead of 21.2 us at 4,096 particles and the force pass 11.7 instead of 14.6.
+// (each line with the other pass fixed). Four lanes per particle in the force
+// (k_force_tra_quad) against that small build: 34.6 / 29.2 at 4,096 particles,
+// 40.4 / 38.7 at 21,952 (4.5), 43.7 / 44.8 at 32,768. Alone, the density pass
+// takes 7.9 instead of 21.2 us at 4,096 particles and the force pass 7.2
+// instead of 14.6.
 constexpr int kRowsMax1 = 5;
 constexpr int kRowsMax3 = 17;
+constexpr int kForceQuadMax = 5;
 constexpr int kForceSmallMax = 27;
 
 // Warps per block of the density and force kernels: 8 by default; each
@@ -818,6 +847,28 @@ k_density_sms(Frame f, DevParams P) {
 }
 
 // -------------------------------------------------------------- force TRA --
+// All candidates of a particle, tested as the reference does.
+template <bool kArt>
+__device__ __forceinline__ void force_scan(const Frame &f, const DevParams &P,
+                                           const SceneGeom &G, const MicroPos &mp,
+                                           const float4 &p, const float4 &pev, ForceAcc &a) {
+    for (int r = 0; r < 9; ++r) {
+        const int ny = mp.cy + (r % 3) - 1;
+        const int nz = mp.cz + (r / 3) - 1;
+        if (ny < 0 || ny >= G.gy || nz < 0 || nz >= G.gz) continue;
+        const int m = G.cbase + mp.cx + G.gx * (ny + G.gy * nz);
+        int begin, end;
+        row_range(f, G, m, mp.cx, mp.lmx, mp.lmx, begin, end);
+        for (int j = begin; j < end; ++j) {
+            const float4 q = f.pos[j];
+            const float rx = p.x - q.x, ry = p.y - q.y, rz = p.z - q.z;
+            const float d2 = sq_dist(rx, ry, rz);
+            if (P.h2 < d2 || kFloatSmall > d2) continue;
+            force_pair<true, kArt>(p, pev, q, f.ev[j], P, a);
+        }
+    }
+}
+
 // The neighbours the density pass found, in the same order (rows in sequence,
 // set bits in increasing candidate index). Each lane stages its 9 (row start,
 // mask) pairs in shared memory and walks all its neighbours in one loop, so
@@ -935,24 +986,121 @@ k_force_tra(Frame f, DevParams P, bool fresh) {
                 force_pair<false, kArt>(p, pev, f.pos[j], f.ev[j], P, a);
             }
         } else {
-            for (int r = 0; r < 9; ++r) {
-                const int ny = mp.cy + (r % 3) - 1;
-                const int nz = mp.cz + (r / 3) - 1;
-                if (ny < 0 || ny >= G.gy || nz < 0 || nz >= G.gz) continue;
-                const int m = G.cbase + mp.cx + G.gx * (ny + G.gy * nz);
-                int begin, end;
-                row_range(f, G, m, mp.cx, mp.lmx, mp.lmx, begin, end);
-                for (int j = begin; j < end; ++j) {
-                    const float4 q = f.pos[j];
-                    const float rx = p.x - q.x, ry = p.y - q.y, rz = p.z - q.z;
-                    const float d2 = sq_dist(rx, ry, rz);
-                    if (P.h2 < d2 || kFloatSmall > d2) continue;
-                    force_pair<true, kArt>(p, pev, q, f.ev[j], P, a);
-                }
-            }
+            force_scan<kArt>(f, P, G, mp, p, pev, a);
         }
         write_force(f, P, self, p, pev, G, a, false);
     }
+}
+
+// The same for the smallest scenes, four lanes per particle: with one lane, a
+// warp alone on its scheduler spends the pass in rounds of neighbour loads.
+// The lanes list the particle's neighbours together, each evaluates every
+// fourth of them (the next round's loads in flight), and the terms change
+// hands through shared memory so that each lane keeps one of the four sums
+// (pressure, viscosity, gradient, laplacian) and adds its terms in neighbour
+// order with k_force_tra's operations: the same bits.
+constexpr int kQuadList = 64;   // neighbours listed; with more the first lane scans
+template <bool kArt>
+__global__ void __launch_bounds__(128)
+k_force_tra_quad(Frame f, DevParams P, bool fresh) {
+    __shared__ int list[4][8][kQuadList];
+    __shared__ __align__(16) float terms[4][8][4][12];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int pl = lane >> 2, s = lane & 3;
+    const int middle = f.ctr->middle;
+    const int base = blockIdx.x * 32 + warp * 8;
+    if (base >= middle) return;   // the whole warp
+    const int idx = base + pl;
+    const bool active = idx < middle;
+    const int at = active ? idx : base;   // idle lanes follow a live particle
+    const int self = f.ctr->any_sms ? f.compact[at] : at;
+    const float4 p = f.pos[self];
+    const float4 pev = f.ev[self];
+    const SceneGeom G = geom_of_particle(f.scenes, self);
+    const MicroPos mp = micro_of(p, P, G);
+    int found = fresh ? f.nbr_flag[at] : -1;
+    const bool listed = found >= 0 && found <= kQuadList;
+    // lane s of the particle lists rows s, s + 4 and s + 8
+    const uint32_t *masks = f.nbr_mask + (size_t(at >> 5) * 9) * 32 + (at & 31);
+    uint32_t mk[3];
+    int start[3], cnt[3];
+    const int own = G.cbase + mp.cx + G.gx * (mp.cy + G.gy * mp.cz);
+    const int left = mp.cx > 0 ? 1 : 0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int r = s + 4 * k;
+        mk[k] = listed && r < 9 ? masks[r * 32] : 0u;
+        cnt[k] = __popc(mk[k]);
+        const int m = mk[k] ? own + G.gx * ((r % 3) - 1 + G.gy * ((r / 3) - 1)) : own;
+        const int s0 = f.cell_start[m - left];
+        const int s1 = f.cell_start[m];
+        const uint32_t xs = f.cell_xslab[m - left];
+        start[k] = s0;
+        if (left && mp.lmx > 0 && xs != kXslabUnknown)
+            start[k] = s0 + min(int((xs >> (10 * (mp.lmx - 1))) & 1023u), s1 - s0);
+    }
+    int ahead = 0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        int incl = cnt[k];
+        int v = __shfl_up_sync(kFull, incl, 1, 4);
+        if (s >= 1) incl += v;
+        v = __shfl_up_sync(kFull, incl, 2, 4);
+        if (s >= 2) incl += v;
+        int o = ahead + incl - cnt[k];
+        ahead += __shfl_sync(kFull, incl, 3, 4);
+        for (uint32_t m = mk[k]; m; m &= m - 1u)
+            list[warp][pl][o++] = start[k] + __ffs(m) - 1;
+    }
+    __syncwarp();
+    const int n = listed ? found : 0;
+    const int rounds = (int(__reduce_max_sync(kFull, unsigned(n))) + 3) >> 2;
+    float *mine = terms[warp][pl][s];
+    // the lane's sum: which vector and which factor of a pair's terms
+    const float *vec = terms[warp][pl][0] + (s == 1 ? 4 : s == 3 ? 8 : 0);
+    const float *fac = terms[warp][pl][0] + (s == 0 ? 3 : s == 1 ? 7 : s == 2 ? 9 : 10);
+    float ax = 0.f, ay = 0.f, az = 0.f;
+    int j = s < n ? list[warp][pl][s] : self;
+    float4 q = f.pos[j], e = f.ev[j];
+    for (int k = 0; k < rounds; ++k) {
+        const bool valid = 4 * k + s < n;
+        const float4 cq = q, ce = e;
+        const int next = 4 * (k + 1) + s;
+        j = next < n ? list[warp][pl][next] : self;
+        q = f.pos[j];
+        e = f.ev[j];
+        const PairTerms t = pair_terms<kArt>(p, pev, cq, ce, P);
+        *reinterpret_cast<float4 *>(mine) =
+            make_float4(t.rx, t.ry, t.rz, valid ? -t.ps : 0.f);
+        *reinterpret_cast<float4 *>(mine + 4) =
+            make_float4(t.ux, t.uy, t.uz, valid ? t.wk : 0.f);
+        *reinterpret_cast<float4 *>(mine + 8) =
+            make_float4(t.lf, valid ? t.gw : 0.f, valid ? t.wh : 0.f, 0.f);
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 v = *reinterpret_cast<const float4 *>(vec + 12 * i);
+            const float w = fac[12 * i];
+            ax = __fmaf_rn(v.x, w, ax);
+            ay = __fmaf_rn(v.y, w, ay);
+            az = __fmaf_rn(v.z, w, az);
+        }
+        __syncwarp();
+    }
+    ForceAcc a;
+    a.px = ax;
+    a.py = ay;
+    a.pz = az;
+    a.vx = __shfl_down_sync(kFull, ax, 1);
+    a.vy = __shfl_down_sync(kFull, ay, 1);
+    a.vz = __shfl_down_sync(kFull, az, 1);
+    a.gx = __shfl_down_sync(kFull, ax, 2);
+    a.gy = __shfl_down_sync(kFull, ay, 2);
+    a.gz = __shfl_down_sync(kFull, az, 2);
+    a.lap = __shfl_down_sync(kFull, ax, 3);
+    if (s != 0 || !active) return;
+    if (!listed) force_scan<kArt>(f, P, G, mp, p, pev, a);   // (the sums are zero)
+    write_force(f, P, self, p, pev, G, a, false);
 }
 
 // -------------------------------------------------------------- force SMS --
@@ -1316,7 +1464,9 @@ void launch_force_w(const Frame &f, const DevParams &P, int num_sms, bool fresh,
                     const LaunchShape &shape, cudaStream_t s, cudaStream_t s_sms) {
     k_force_sms<kArt, W><<<num_sms * shape.force_sms, W * 32, 0, s_sms>>>(f, P);
     const int units = (f.n + 31) / 32;
-    if (units <= num_sms * kForceSmallMax)
+    if (units <= num_sms * kForceQuadMax)
+        k_force_tra_quad<kArt><<<units, 128, 0, s>>>(f, P, fresh);
+    else if (units <= num_sms * kForceSmallMax)
         k_force_tra<kArt, 2, true><<<(units + 1) / 2, 64, 0, s>>>(f, P, fresh);
     else
         k_force_tra<kArt, W><<<num_sms * shape.force_tra, W * 32, 0, s>>>(f, P, fresh);

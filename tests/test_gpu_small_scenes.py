@@ -1,10 +1,11 @@
 """The TRA passes choose among builds by the number of particles: density with
 a work unit's rows spread over nine or three warps or walked by one, force with
-two or four neighbours in flight. A scene gives the same bits whichever runs:
+four lanes per particle, or with four or two neighbours in flight. A scene gives the same bits whichever runs:
 alone (a small-scene build) and in a batch large enough for the general ones.
 Sizes sit around the rules' lines (units per SM times 152 SMs times 32
 particles); the crowded scenes have rows of more than 32 candidates (no mask)
-and more than 12 interacting ones (past the terms kept in shared memory)."""
+and more than 12 interacting ones (past the terms kept in shared memory), and
+particles with more than 64 neighbours (past the four lanes' list)."""
 import numpy as np
 import pytest
 
@@ -29,7 +30,7 @@ def state(gsph, sysm, all_tra):
 
 
 CASES = {   # particles, positions pulled together by
-    "one": (1, 1.0), "unit-1": (31, 1.0), "unit+1": (33, 1.0), "odd": (1501, 1.0),
+    "one": (1, 1.0), "quad+1": (9, 1.0), "unit-1": (31, 1.0), "unit+1": (33, 1.0), "odd": (1501, 1.0),
     "row-per-warp": (24320, 1.0), "three-rows": (24321, 1.0), "force-line": (82689, 1.0),
     "crowded": (2000, 0.6), "very crowded": (2000, 0.2), "crowded, three rows": (30000, 0.3),
 }
