@@ -139,8 +139,9 @@ __device__ __forceinline__ float artificial_pair(float vr, float d2, float k,
                                                  float inv_d, float vi, float vj,
                                                  const DevParams &P) {
     if (!(vr < 0.f)) return 0.f;
-    const float mu = __fdividef(P.h * vr, d2 + P.art_eps);
-    const float pij = __fdividef(-2.f * P.art_coef * mu * vi * vj, vi + vj);
+    // mu and the mean density's reciprocal under one division
+    const float num = -2.f * P.art_coef * P.h * vr * vi * vj;
+    const float pij = __fdividef(num, (d2 + P.art_eps) * (vi + vj));
     return pij * k * k * inv_d;
 }
 
@@ -1162,6 +1163,10 @@ k_force_sms(Frame f, DevParams P) {
         // gradient is accumulated with the opposite sign and negated at the end
         float2 Px = zero, Py = zero, Pz = zero, Vx = zero, Vy = zero, Vz = zero;
         float2 Gx = zero, Gy = zero, Gz = zero, L = zero, S = zero;
+        // artificial viscosity: -2 alpha c0 h V_i, V_i and 0.01 h^2
+        const float art = -2.f * P.art_coef * P.h * p.w;
+        const float2 artv = make_float2(art, art), viv = make_float2(p.w, p.w);
+        const float2 epsv = make_float2(P.art_eps, P.art_eps);
         // added to r^2 so that 1/r stays finite for the particle itself, whose
         // terms are zeroed; far below a rounding of any interacting r^2
         const float2 tiny = make_float2(1e-30f, 1e-30f);
@@ -1215,9 +1220,16 @@ k_force_sms(Frame f, DevParams P) {
                         float2 vr = __fmul2_rn(dvx, dx);
                         vr = __ffma2_rn(dvy, dy, vr);
                         vr = __ffma2_rn(dvz, dz, vr);
-                        const float2 w = make_float2(
-                            okx ? artificial_pair(vr.x, d2.x, kk.x, inv.x, p.w, qb.z, P) : 0.f,
-                            oky ? artificial_pair(vr.y, d2.y, kk.y, inv.y, p.w, qb.w, P) : 0.f);
+                        // artificial_pair, packed; V is zero where the pair
+                        // does not interact
+                        const float2 vn = make_float2(fminf(vr.x, 0.f), fminf(vr.y, 0.f));
+                        const float2 den =
+                            __fmul2_rn(__fadd2_rn(d2, epsv),
+                                       __fadd2_rn(make_float2(qb.z, qb.w), viv));
+                        const float2 rcp =
+                            make_float2(__fdividef(1.f, den.x), __fdividef(1.f, den.y));
+                        float2 w = __fmul2_rn(__fmul2_rn(__fmul2_rn(vn, V), artv), rcp);
+                        w = __fmul2_rn(__fmul2_rn(__fmul2_rn(w, kk), kk), inv);
                         Vx = __ffma2_rn(dx, w, Vx);
                         Vy = __ffma2_rn(dy, w, Vy);
                         Vz = __ffma2_rn(dz, w, Vz);
