@@ -342,6 +342,18 @@ gsph_status check_grid(const gsph_params &p, const char *who, long long *numc);
 SceneGeom make_scene_geom(const gsph_params &p, int cbase);
 void set_error(const char *fmt, ...);
 
+// The scene server's data path (system.cu): gsph_batch_repack with each new
+// scene's arrays where they lie (vel4 may be null: zero), and the final
+// positions and velocities of several scenes with one wait.
+struct SceneArrays {
+    const float *pos4, *vel4;
+};
+gsph_status batch_repack_from(gsph_handle h, const uint32_t *keep, uint32_t n_keep,
+                              const gsph_params *add_params, const uint32_t *add_counts,
+                              uint32_t n_add, const SceneArrays *add);
+gsph_status batch_read_scenes(gsph_handle h, const uint32_t *scenes, uint32_t count,
+                              float *const *pos4, float *const *vel4);
+
 // Snapshot file format (snapshot.cpp).
 gsph_status snapshot_write(const char *path, const gsph_params *plist,
                            const uint32_t *counts, uint32_t n_scenes,

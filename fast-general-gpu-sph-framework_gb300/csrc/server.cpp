@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <cstring>
 #include <deque>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <unordered_map>
@@ -37,10 +38,20 @@ void fail(const char *msg) { gsph::set_error("%s", msg); }
 constexpr uint64_t kBytesPerParticle = 221;
 constexpr uint64_t kBytesPerCell = 44;
 
+// A host array without a first pass that zeroes it (every one is filled whole).
+struct HostArray {
+    std::unique_ptr<float[]> data;
+    bool alloc(size_t count) {
+        data.reset(count ? new (std::nothrow) float[count] : nullptr);
+        return !count || data;
+    }
+    const float *get() const { return data.get(); }
+};
+
 struct Request {
     uint64_t id = 0;
     gsph_params params{};
-    std::vector<float> pos, vel;   // float4 per particle
+    HostArray pos, vel;   // float4 per particle; vel empty: zero
     uint32_t n = 0;
     uint64_t cells = 0;
     uint32_t frames = 0;
@@ -132,13 +143,13 @@ gsph_status gsph_server_submit(gsph_server_handle s, uint64_t id, const gsph_par
     r.n = n;
     r.cells = cells_of(*p);
     r.frames = r.remaining = frames;
-    try {
-        r.pos.assign(pos4, pos4 + size_t(n) * 4);
-        if (vel4) r.vel.assign(vel4, vel4 + size_t(n) * 4);
-    } catch (...) {
+    const size_t floats = size_t(n) * 4;
+    if (!r.pos.alloc(floats) || (vel4 && !r.vel.alloc(floats))) {
         fail("gsph_server_submit: host allocation failed");
         return GSPH_ERR_OUT_OF_MEMORY;
     }
+    if (floats) std::memcpy(r.pos.data.get(), pos4, floats * sizeof(float));
+    if (floats && vel4) std::memcpy(r.vel.data.get(), vel4, floats * sizeof(float));
     std::lock_guard<std::mutex> lock(s->mu);
     s->queue.push_back(std::move(r));
     ++s->stats.submitted;
@@ -158,31 +169,32 @@ struct ShardPlan {
 gsph_status apply_plan(const gsph_server_config &cfg, Shard &sh, ShardPlan &pl) {
     std::vector<gsph_params> plist;
     std::vector<uint32_t> counts;
-    std::vector<float> pos, vel;
-    bool any_vel = false;
-    for (const Request &r : pl.admitted) any_vel |= !r.vel.empty();
+    std::vector<gsph::SceneArrays> add;
     for (const Request &r : pl.admitted) {
         plist.push_back(r.params);
         counts.push_back(r.n);
-        pos.insert(pos.end(), r.pos.begin(), r.pos.end());
-        if (any_vel) {
-            if (r.vel.empty())
-                vel.insert(vel.end(), size_t(r.n) * 4, 0.f);
-            else
-                vel.insert(vel.end(), r.vel.begin(), r.vel.end());
-        }
+        add.push_back({r.pos.get(), r.vel.get()});
     }
-    if (!sh.batch)
-        return gsph_batch_create_ex(plist.data(), counts.data(), uint32_t(plist.size()),
-                                    pos.empty() ? nullptr : pos.data(),
-                                    any_vel ? vel.data() : nullptr, cfg.particle_capacity,
-                                    cfg.cell_capacity, cfg.scene_capacity, cfg.device,
-                                    &sh.batch);
-    return gsph_batch_repack(sh.batch, pl.keep.empty() ? nullptr : pl.keep.data(),
-                             uint32_t(pl.keep.size()), plist.empty() ? nullptr : plist.data(),
-                             counts.empty() ? nullptr : counts.data(), uint32_t(plist.size()),
-                             pos.empty() ? nullptr : pos.data(),
-                             any_vel ? vel.data() : nullptr);
+    if (sh.batch)
+        return gsph::batch_repack_from(sh.batch, pl.keep.data(), uint32_t(pl.keep.size()),
+                                       plist.data(), counts.data(), uint32_t(plist.size()),
+                                       add.data());
+    // the batch's first scenes: gsph_batch_create_ex takes them concatenated
+    std::vector<float> pos, vel;
+    bool any_vel = false;
+    for (const Request &r : pl.admitted) any_vel |= bool(r.vel.data);
+    for (const Request &r : pl.admitted) {
+        const size_t floats = size_t(r.n) * 4;
+        pos.insert(pos.end(), r.pos.get(), r.pos.get() + floats);
+        if (any_vel && r.vel.data)
+            vel.insert(vel.end(), r.vel.get(), r.vel.get() + floats);
+        else if (any_vel)
+            vel.insert(vel.end(), floats, 0.f);
+    }
+    return gsph_batch_create_ex(plist.data(), counts.data(), uint32_t(plist.size()),
+                                pos.empty() ? nullptr : pos.data(),
+                                any_vel ? vel.data() : nullptr, cfg.particle_capacity,
+                                cfg.cell_capacity, cfg.scene_capacity, cfg.device, &sh.batch);
 }
 
 }  // namespace
@@ -276,10 +288,8 @@ gsph_status gsph_server_step(gsph_server_handle s, int *frames_stepped) {
         next.reserve(pl.keep.size() + pl.admitted.size());
         for (uint32_t k : pl.keep) next.push_back(std::move(sh.resident[k]));
         for (Request &r : pl.admitted) {
-            r.pos.clear();
-            r.pos.shrink_to_fit();
-            r.vel.clear();
-            r.vel.shrink_to_fit();
+            r.pos.data.reset();
+            r.vel.data.reset();
             next.push_back(std::move(r));
         }
         sh.resident = std::move(next);
@@ -309,6 +319,8 @@ gsph_status gsph_server_step(gsph_server_handle s, int *frames_stepped) {
     }
     std::vector<Request> done;
     for (Shard &sh : s->shards) {   // resident lists change only on this thread
+        std::vector<uint32_t> scenes;
+        std::vector<float *> pos, vel;
         for (size_t i = 0; i < sh.resident.size(); ++i) {
             const Request &r = sh.resident[i];
             if (r.remaining) continue;
@@ -317,17 +329,19 @@ gsph_status gsph_server_step(gsph_server_handle s, int *frames_stepped) {
             out.params = r.params;
             out.n = r.n;
             out.frames = r.frames;
-            out.pos.resize(size_t(r.n) * 4);
-            out.vel.resize(size_t(r.n) * 4);
-            if (r.n) {
-                if ((st = gsph_copy_out_scene(sh.batch, uint32_t(i), GSPH_FIELD_POSITION,
-                                              out.pos.data(), out.pos.size() * 4)) ||
-                    (st = gsph_copy_out_scene(sh.batch, uint32_t(i), GSPH_FIELD_VELOCITY,
-                                              out.vel.data(), out.vel.size() * 4)))
-                    return st;
+            if (!out.pos.alloc(size_t(r.n) * 4) || !out.vel.alloc(size_t(r.n) * 4)) {
+                fail("gsph_server_step: host allocation failed");
+                return GSPH_ERR_OUT_OF_MEMORY;
             }
+            scenes.push_back(uint32_t(i));
+            pos.push_back(out.pos.data.get());
+            vel.push_back(out.vel.data.get());
             done.push_back(std::move(out));
         }
+        if (!scenes.empty() &&
+            (st = gsph::batch_read_scenes(sh.batch, scenes.data(), uint32_t(scenes.size()),
+                                          pos.data(), vel.data())))
+            return st;
     }
     std::lock_guard<std::mutex> lock(s->mu);
     for (Request &r : done) {
@@ -370,10 +384,9 @@ gsph_status gsph_server_take(gsph_server_handle s, uint64_t id, float *pos4, flo
         fail("gsph_server_take: request not finished or already taken");
         return GSPH_ERR_STATE;
     }
-    if (pos4 && !it->second.pos.empty())
-        std::memcpy(pos4, it->second.pos.data(), it->second.pos.size() * sizeof(float));
-    if (vel4 && !it->second.vel.empty())
-        std::memcpy(vel4, it->second.vel.data(), it->second.vel.size() * sizeof(float));
+    const size_t bytes = size_t(it->second.n) * 4 * sizeof(float);
+    if (pos4 && bytes) std::memcpy(pos4, it->second.pos.get(), bytes);
+    if (vel4 && bytes) std::memcpy(vel4, it->second.vel.get(), bytes);
     s->finished.erase(it);
     return GSPH_OK;
 }

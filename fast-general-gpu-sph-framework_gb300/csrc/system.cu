@@ -96,6 +96,7 @@ struct System {
     float4 *acc = nullptr;
     int cur = 0;   // buffer index that holds the current (sorted) state
     Frame fr{};    // pointers shared by both parities
+    Counters *host_ctr = nullptr;   // pinned
     double *red = nullptr;   // reductions workspace
     bool arranged = false;   // sorted state + split valid
     bool grid_current = false;   // no position changed since the last arrange
@@ -193,6 +194,10 @@ struct System {
         xfer_pending = false;
         for (void *p : allocs) cudaFree(p);
         allocs.clear();
+        if (host_ctr) {
+            cudaFreeHost(host_ctr);
+            host_ctr = nullptr;
+        }
         if (stream) {
             cudaStreamDestroy(stream);
             stream = nullptr;
@@ -326,6 +331,7 @@ struct System {
         GSPH_CUDA(cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking));
         GSPH_CUDA(cudaEventCreateWithFlags(&fork_ev, cudaEventDisableTiming));
         GSPH_CUDA(cudaEventCreateWithFlags(&join_ev, cudaEventDisableTiming));
+        GSPH_CUDA(cudaMallocHost(reinterpret_cast<void **>(&host_ctr), sizeof(Counters)));
         long long n_total = 0, c_total = 0;
         if (count < 1) {
             set_error("a batch needs at least one scene at creation");
@@ -400,8 +406,7 @@ struct System {
     // followed by new ones. The kept scenes' state is copied on the device
     // in its current order, so each continues exactly as if alone.
     gsph_status repack(const uint32_t *keep, int n_keep, const gsph_params *add_p,
-                       const uint32_t *add_n, int n_add, const float *add_pos4,
-                       const float *add_vel4) {
+                       const uint32_t *add_n, int n_add, const SceneArrays *add) {
         const int S_old = int(geom.size());
         std::vector<gsph_params> plist;
         std::vector<uint32_t> counts;
@@ -468,19 +473,31 @@ struct System {
                 d_repack + n_keep + 1, n_keep, kept_total);
             GSPH_CUDA(cudaGetLastError());
         }
-        // new scenes: contiguous after the kept ones, one copy per array
+        // new scenes: contiguous after the kept ones; scenes that lie one after
+        // another in host memory too go up in one copy per array
         const size_t added = size_t(n_total - kept_total);
         if (added > 0) {
-            GSPH_CUDA(cudaMemcpyAsync(pos[dst] + kept_total, add_pos4,
-                                      sizeof(float4) * added, cudaMemcpyHostToDevice,
-                                      stream));
-            if (add_vel4)
-                GSPH_CUDA(cudaMemcpyAsync(vel[dst] + kept_total, add_vel4,
-                                          sizeof(float4) * added,
-                                          cudaMemcpyHostToDevice, stream));
-            else
-                GSPH_CUDA(cudaMemsetAsync(vel[dst] + kept_total, 0,
-                                          sizeof(float4) * added, stream));
+            auto upload = [&](float4 *to, const float *SceneArrays::*src) -> gsph_status {
+                for (int k = 0; k < n_add;) {
+                    const float *from = add[k].*src;
+                    size_t len = add_n[k];
+                    int next = k + 1;
+                    while (next < n_add && (from ? add[next].*src == from + 4 * len
+                                                 : !(add[next].*src)))
+                        len += add_n[next++];
+                    if (len && from)
+                        GSPH_CUDA(cudaMemcpyAsync(to, from, sizeof(float4) * len,
+                                                  cudaMemcpyHostToDevice, stream));
+                    else if (len)
+                        GSPH_CUDA(cudaMemsetAsync(to, 0, sizeof(float4) * len, stream));
+                    to += len;
+                    k = next;
+                }
+                return GSPH_OK;
+            };
+            if ((st = upload(pos[dst] + kept_total, &SceneArrays::pos4)) ||
+                (st = upload(vel[dst] + kept_total, &SceneArrays::vel4)))
+                return st;
             GSPH_CUDA(cudaMemsetAsync(ev[dst] + kept_total, 0, sizeof(float4) * added,
                                       stream));
         }
@@ -698,19 +715,22 @@ struct System {
         return GSPH_OK;
     }
 
+    // Waits for the stream and returns the counters: one copy into pinned
+    // memory behind the stream's work, one wait.
     gsph_status read_counters(Counters &c) {
-        GSPH_CUDA(cudaMemcpyAsync(&c, fr.ctr, sizeof(Counters),
+        GSPH_CUDA(cudaMemcpyAsync(host_ctr, fr.ctr, sizeof(Counters),
                                   cudaMemcpyDeviceToHost, stream));
         GSPH_CUDA(cudaStreamSynchronize(stream));
+        c = *host_ctr;
         return GSPH_OK;
     }
 
-    gsph_status sync_and_check() {
+    gsph_status sync_and_check(Counters *out = nullptr) {
         join_xfer();
-        GSPH_CUDA(cudaStreamSynchronize(stream));
         Counters c;
         gsph_status st = read_counters(c);
         if (st) return st;
+        if (out) *out = c;
         if (c.err & kErrOutOfDomain) {
             set_error("a particle left the simulation grid (first index %d); it "
                       "was clamped into the boundary cell",
@@ -954,6 +974,43 @@ float4 *state_ptr(System &s, gsph_field f) {
 
 }  // namespace
 
+namespace gsph {
+
+gsph_status batch_repack_from(gsph_handle h, const uint32_t *keep, uint32_t n_keep,
+                              const gsph_params *add_params, const uint32_t *add_counts,
+                              uint32_t n_add, const SceneArrays *add) {
+    gsph_status st = check_handle(h);
+    if (st) return st;
+    System &s = h->sys;
+    GSPH_CUDA(cudaStreamSynchronize(s.stream));
+    return s.repack(keep, int(n_keep), add_params, add_counts, int(n_add), add);
+}
+
+gsph_status batch_read_scenes(gsph_handle h, const uint32_t *scenes, uint32_t count,
+                              float *const *pos4, float *const *vel4) {
+    gsph_status st = check_handle(h);
+    if (st) return st;
+    System &s = h->sys;
+    if ((st = s.sync_and_check()) && st != GSPH_ERR_DOMAIN) return st;
+    for (uint32_t k = 0; k < count; ++k) {
+        if (scenes[k] >= s.geom.size()) {
+            set_error("batch_read_scenes: scene %u out of range", scenes[k]);
+            return GSPH_ERR_INVALID_ARG;
+        }
+        const int p0 = s.pbase[scenes[k]];
+        const size_t bytes = sizeof(float4) * size_t(s.pbase[scenes[k] + 1] - p0);
+        if (!bytes) continue;
+        GSPH_CUDA(cudaMemcpyAsync(pos4[k], s.pos[s.cur] + p0, bytes, cudaMemcpyDeviceToHost,
+                                  s.stream));
+        GSPH_CUDA(cudaMemcpyAsync(vel4[k], s.vel[s.cur] + p0, bytes, cudaMemcpyDeviceToHost,
+                                  s.stream));
+    }
+    GSPH_CUDA(cudaStreamSynchronize(s.stream));
+    return GSPH_OK;
+}
+
+}  // namespace gsph
+
 extern "C" {
 
 gsph_status gsph_create(const gsph_params *p, const float *pos4,
@@ -1134,10 +1191,14 @@ gsph_status gsph_batch_repack(gsph_handle h, const uint32_t *keep, uint32_t n_ke
         set_error("gsph_batch_repack: null positions");
         return GSPH_ERR_INVALID_ARG;
     }
-    System &s = h->sys;
-    GSPH_CUDA(cudaStreamSynchronize(s.stream));
-    return s.repack(keep, int(n_keep), add_params, add_counts, int(n_add), add_pos4,
-                    add_vel4);
+    std::vector<SceneArrays> add;
+    const float *pos = add_pos4, *vel = add_vel4;
+    for (uint32_t k = 0; k < n_add; ++k) {
+        add.push_back({pos, vel});
+        if (pos) pos += size_t(add_counts[k]) * 4;
+        if (vel) vel += size_t(add_counts[k]) * 4;
+    }
+    return batch_repack_from(h, keep, n_keep, add_params, add_counts, n_add, add.data());
 }
 
 gsph_status gsph_destroy(gsph_handle h) {
@@ -1267,9 +1328,8 @@ gsph_status gsph_copy_out(gsph_handle h, gsph_field field, void *host_dst,
         return GSPH_ERR_INVALID_ARG;
     }
     System &s = h->sys;
-    if ((st = s.sync_and_check()) && st != GSPH_ERR_DOMAIN) return st;
     Counters c;
-    if ((st = s.read_counters(c))) return st;
+    if ((st = s.sync_and_check(&c)) && st != GSPH_ERR_DOMAIN) return st;
     const int T = s.arranged ? c.task_count : 0;
     if (field == GSPH_FIELD_TASKS) {
         const size_t need = size_t(T + (T & 1)) * sizeof(gsph_block_task);
