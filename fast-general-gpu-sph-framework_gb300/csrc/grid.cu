@@ -179,6 +179,22 @@ k_cell_scan(const int32_t *__restrict__ count, int numc,
     __syncthreads();
     unsigned long long run = x - s;
     for (int w = 0; w < kScanThreads / 32; ++w) run += wb[w] + (w < warp ? ws[w] : 0ull);
+    // places for the thread's large cells: one atomic per warp that has any
+    int big = 0;
+#pragma unroll
+    for (int q = 0; q < kScanItems; ++q) big += v[q] > kSmallCellMax ? 1 : 0;
+    int big_at = 0;
+    if (__any_sync(kFull, big > 0)) {
+        int incl = big;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += y;
+        }
+        int base = 0;
+        if (lane == 31) base = atomicAdd(&ctr->big_fill, incl);
+        big_at = __shfl_sync(kFull, base, 31) + incl - big;
+    }
     int out[kScanItems];
 #pragma unroll
     for (int q = 0; q < kScanItems; ++q) {
@@ -186,8 +202,7 @@ k_cell_scan(const int32_t *__restrict__ count, int numc,
         out[q] = int32_t(run & 0xFFFFFFFFull);
         if (c < numc && v[q] > 0) {
             occ_list[run >> 32] = c;
-            if (v[q] > kSmallCellMax)
-                big_list[atomicAdd(&ctr->big_fill, 1)] = int32_t(run >> 32);
+            if (v[q] > kSmallCellMax) big_list[big_at++] = int32_t(run >> 32);
         }
         run += pack_cell(v[q]);
     }
