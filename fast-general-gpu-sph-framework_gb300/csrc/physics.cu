@@ -626,10 +626,14 @@ __device__ __forceinline__ ClusterBox cluster_box(const float4 &p, uint32_t key)
 // 128); else they come from the queue. Negative: done.
 struct ClusterUnits {
     int count, per, own;
-    __device__ __forceinline__ ClusterUnits(int units, int warps) : count(units) {
-        per = (units + int(gridDim.x) - 1) / int(gridDim.x);
+    // blocks: those of the grid that run at once
+    __device__ __forceinline__ ClusterUnits(int units, int warps, int blocks)
+        : count(units) {
+        per = (units + blocks - 1) / blocks;
         const int warp = threadIdx.x >> 5;
-        own = per > warps ? -2 : warp < per ? int(blockIdx.x) * per + warp : -1;
+        own = per > warps ? -2
+              : warp < per && int(blockIdx.x) < blocks ? int(blockIdx.x) * per + warp
+                                                       : -1;
     }
     __device__ __forceinline__ int next(int *queue) {
         int u = own;
@@ -815,7 +819,7 @@ k_density_sms(Frame f, DevParams P) {
     float4 *sxy = sms_xy[warp];
     float2 *szz = sms_zz[warp];
     const int i = lane % C, g = lane / C;
-    ClusterUnits units(task_count * kGroups, W);
+    ClusterUnits units(task_count * kGroups, W, gridDim.x);
     for (int u; (u = units.next(&f.ctr->work_density_sms)) >= 0;) {
         const gsph_block_task task = f.tasks[u / kGroups];
         const int first = task.cell_begin + task_offset(task) + (u % kGroups) * C;
@@ -1135,10 +1139,11 @@ k_force_tra_quad(Frame f, DevParams P, bool fresh) {
 // expression; the two halves of every accumulator and then the groups' sums
 // are added at the end.
 constexpr int kForceCluster = 16;
+static_assert(kForceCluster == kDenCluster, "sms_blocks counts one cluster size");
 constexpr int kForceSmsCtas = 3;   // resident blocks per SM
 template <bool kArt, int W>
 __global__ void __launch_bounds__(W * 32, kForceSmsCtas * kWarpsPerBlock / W)
-k_force_sms(Frame f, DevParams P) {
+k_force_sms(Frame f, DevParams P, int resident) {
     constexpr int C = kForceCluster, kGroups = 32 / C;
     // candidate pair k (slots 2k, 2k+1) as four float4s: (x, x, y, y),
     // (z, z, 1/rho, 1/rho), (vx, vx, vy, vy), (vz, vz, p, p)
@@ -1150,7 +1155,7 @@ k_force_sms(Frame f, DevParams P) {
     if (task_count == 0) return;   // no SMS work: skip the queue atomics
     float4 *sa = sm[0][warp], *sb4 = sm[1][warp], *sc = sm[2][warp], *sd = sm[3][warp];
     const int i = lane % C, g = lane / C;
-    ClusterUnits units(task_count * kGroups, W);
+    ClusterUnits units(task_count * kGroups, W, min(int(gridDim.x), resident));
     for (int u; (u = units.next(&f.ctr->work_force_sms)) >= 0;) {
         const gsph_block_task task = f.tasks[u / kGroups];
         const int first = task.cell_begin + task_offset(task) + (u % kGroups) * C;
@@ -1474,11 +1479,22 @@ cudaError_t configure_shape(int smem) {
     return set_carveout(k_force_sms<true, W>, kForceSmsCtas * k, smem, W * 32);
 }
 
+// Blocks of an SMS pass: `ctas` per SM, but one or two where the scene's
+// clusters cannot fill more. (All-TRA frames, whose SMS blocks only look and
+// leave, feel the difference: 13,824 particles 33.7 us a frame with four per
+// SM, 32.6 with one. Three, which fill the SMs' shared memory to the last
+// block, hold the TRA blocks back: 39.9.)
+int sms_blocks(const Frame &f, int num_sms, int ctas, int warps) {
+    const int clusters = f.n / kDenCluster + 1;
+    const int need = (clusters + num_sms * warps - 1) / (num_sms * warps);
+    return num_sms * (need <= 2 ? std::min(need, ctas) : ctas);
+}
+
 template <int W>
 void launch_density_w(const Frame &f, const DevParams &P, int num_sms,
                       const LaunchShape &shape, cudaStream_t s, cudaStream_t s_sms,
                       bool row_prefetch) {
-    k_density_sms<W><<<num_sms * shape.density_sms, W * 32, 0, s_sms>>>(f, P);
+    k_density_sms<W><<<sms_blocks(f, num_sms, shape.density_sms, W), W * 32, 0, s_sms>>>(f, P);
     const int units = (f.n + 31) / 32;
     if (units <= num_sms * kRowsMax1)
         launch_after(k_density_tra_rows<1>, units, 288, s, f, P);
@@ -1493,9 +1509,8 @@ void launch_density_w(const Frame &f, const DevParams &P, int num_sms,
 template <bool kArt, int W>
 void launch_force_w(const Frame &f, const DevParams &P, int num_sms, bool fresh,
                     const LaunchShape &shape, cudaStream_t s, cudaStream_t s_sms) {
-    // (a tuned shape may ask for more blocks than are resident)
-    const int ctas = std::min(shape.force_sms, kForceSmsCtas * kWarpsPerBlock / W);
-    k_force_sms<kArt, W><<<num_sms * ctas, W * 32, 0, s_sms>>>(f, P);
+    k_force_sms<kArt, W><<<sms_blocks(f, num_sms, shape.force_sms, W), W * 32, 0, s_sms>>>(
+        f, P, num_sms * kForceSmsCtas * kWarpsPerBlock / W);
     const int units = (f.n + 31) / 32;
     if (units <= num_sms * kForceQuadMax)
         k_force_tra_quad<kArt><<<units, 128, 0, s>>>(f, P, fresh);
