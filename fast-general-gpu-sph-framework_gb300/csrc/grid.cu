@@ -128,20 +128,55 @@ k_tile_sums(const int32_t *__restrict__ count, int numc,
     }
 }
 
-// The scan, one tile per CTA; a CTA adds up what lies before its tile itself:
-// the sums of the earlier tiles (at most 16,384 of them, read from L2) or, in
-// the direct build, their counts, which for up to kScanDirectTiles tiles takes
-// less time than the launch of k_tile_sums (frame of 13,824 particles, 4 tiles,
-// 39.1 against 40.2 us; of 46,656, 13 tiles, 58.3 against 55.9). (Tile sums kept by the hash's
-// atomics instead need no pass at all, but contend: hash 24 -> 236 us for
-// 3.94M particles in 38 tiles.) The last tile's CTA writes the grand total and
+// Exclusive scan of the tile sums, in place, by one block of 1,024 threads.
+__global__ void __launch_bounds__(1024)
+k_scan_tiles(unsigned long long *__restrict__ tiles, int ntiles) {
+    chain_wait();
+    chain_next();
+    __shared__ unsigned long long ws[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned long long carry = 0;
+    for (int base = 0; base < ntiles; base += 1024) {
+        const int t = base + threadIdx.x;
+        const unsigned long long v = t < ntiles ? tiles[t] : 0ull;
+        unsigned long long x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(kFull, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) ws[warp] = x;
+        __syncthreads();
+        unsigned long long w = ws[lane];   // every warp scans the 32 warp sums
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(kFull, w, o);
+            if (lane >= o) w += y;
+        }
+        const unsigned long long before = __shfl_sync(kFull, w, warp > 0 ? warp - 1 : 0);
+        if (t < ntiles) tiles[t] = carry + (warp > 0 ? before : 0ull) + x - v;
+        carry += __shfl_sync(kFull, w, 31);
+        __syncthreads();
+    }
+}
+
+// The scan, one tile per CTA; a CTA adds up what lies before its tile itself.
+// kBefore says from what: the earlier tiles' counts, which for a few tiles
+// takes less time than the launch of k_tile_sums (frame of 13,824 particles, 8
+// tiles, 39.1 against 40.2 us; of 46,656, 26 tiles, 58.3 against 55.9); the
+// earlier tiles' sums; or, with so many tiles that every CTA reading them all
+// shows (9,216 tiles: 4,345 against 4,339 us a frame, growing as the square),
+// the scanned sums. (Tile sums kept by the hash's atomics
+// instead need no pass at all, but contend: hash 24 -> 236 us for 3.94M
+// particles in 38 tiles.) The last tile's CTA writes the grand total and
 // resets the frame's counters.
-template <bool kDirect>
+enum class Before { kCounts, kSums, kScanned };
+template <Before kBefore>
 __global__ void __launch_bounds__(kScanThreads)
 k_cell_scan(const int32_t *__restrict__ count, int numc,
             const unsigned long long *__restrict__ tiles,
             int32_t *__restrict__ cell_start, int32_t *__restrict__ occ_list,
-            int32_t *__restrict__ big_list, Counters *ctr, int n_particles) {
+            int32_t *__restrict__ big_list, Counters *ctr, int n_particles, int crowd) {
     chain_wait();
     chain_next();
     const int first = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
@@ -151,7 +186,7 @@ k_cell_scan(const int32_t *__restrict__ count, int numc,
 #pragma unroll
     for (int q = 0; q < kScanItems; ++q) s += pack_cell(v[q]);
     unsigned long long before = 0;
-    if (kDirect) {
+    if (kBefore == Before::kCounts) {
         const int4 *c4 = reinterpret_cast<const int4 *>(count);
         int cnt = 0, occ = 0;
 #pragma unroll 8
@@ -161,8 +196,10 @@ k_cell_scan(const int32_t *__restrict__ count, int numc,
             occ += min(c.x, 1) + min(c.y, 1) + min(c.z, 1) + min(c.w, 1);
         }
         before = ((unsigned long long)(unsigned)occ << 32) | (unsigned)cnt;
-    } else {
+    } else if (kBefore == Before::kSums) {
         for (int t = threadIdx.x; t < int(blockIdx.x); t += kScanThreads) before += tiles[t];
+    } else if (threadIdx.x == 0) {
+        before = tiles[blockIdx.x];
     }
     // block exclusive scan of per-thread sums, and the sum of `before`
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -195,6 +232,10 @@ k_cell_scan(const int32_t *__restrict__ count, int numc,
         if (lane == 31) base = atomicAdd(&ctr->big_fill, incl);
         big_at = __shfl_sync(kFull, base, 31) + incl - big;
     }
+    int most = 0;
+#pragma unroll
+    for (int q = 0; q < kScanItems; ++q) most = max(most, v[q]);
+    if (__any_sync(kFull, most >= crowd) && lane == 0) atomicOr(&ctr->crowded, 1);
     int out[kScanItems];
 #pragma unroll
     for (int q = 0; q < kScanItems; ++q) {
@@ -237,12 +278,14 @@ k_cell_scan(const int32_t *__restrict__ count, int numc,
 // `model_blocks` blocks of the performance model, which like the scatter
 // needs nothing but the cell offsets: in small scenes the two overlap (4,096
 // particles 5.2 us against 2.9 + 5.5 as two launches; 3.94M 23.7 against 12.6
-// + 10.3). Also publishes the number of large cells.
+// + 10.3). The model is skipped where the scan saw no cell crowded enough for
+// the SMS path (3.94M 23.7 -> 18.8 us). Also publishes the number of large cells.
 __global__ void __launch_bounds__(kScanThreads)
 k_scatter(Frame f, DevParams P, int model_blocks) {
     chain_wait();
     chain_next();
     if (int(blockIdx.x) < model_blocks) {
+        if (!f.ctr->crowded) return;   // no cell can take the SMS path
         const int num_occ = f.ctr->num_occ;
         for (int tile = blockIdx.x; tile * kValTile < num_occ; tile += model_blocks)
             model_tile(f, P, tile, num_occ);
@@ -343,6 +386,7 @@ __global__ void __launch_bounds__(256) k_sort_small(Frame f) {
     int block = blockIdx.x;
     if (f.cell_val && block-- == 0) {
         model_totals(f);
+        if (threadIdx.x == 0) f.ctr->crowded = 0;   // for the next cell scan
         return;
     }
     int s[2];
@@ -609,15 +653,27 @@ void launch_hash_count(const Frame &f, const DevParams &P, cudaStream_t s) {
 
 void launch_cell_scan(const Frame &f, const DevParams &P, cudaStream_t s) {
     const int ntiles = (P.numc + kScanTile - 1) / kScanTile;
+    // with every count below this a cell's own count is below sparse_self and
+    // the seven counts the model adds up are below sparse_total together
+    const int crowd = std::min(P.sparse_self, P.sparse_total / 7 + (P.sparse_total % 7 > 0));
+    auto scan = [&](auto kernel) {
+        launch_after(kernel, ntiles, kScanThreads, s, f.cell_count, P.numc, f.scan_tiles,
+                     f.cell_start, f.occ_list, f.big_list, f.ctr, f.n, crowd);
+    };
     if (ntiles <= kScanDirectTiles) {
-        k_cell_scan<true><<<ntiles, kScanThreads, 0, s>>>(f.cell_count, P.numc, nullptr,
-                                                          f.cell_start, f.occ_list,
-                                                          f.big_list, f.ctr, f.n);
+        // an ordinary launch: what precedes it in the stream need not be a kernel
+        k_cell_scan<Before::kCounts><<<ntiles, kScanThreads, 0, s>>>(
+            f.cell_count, P.numc, nullptr, f.cell_start, f.occ_list, f.big_list, f.ctr, f.n,
+            crowd);
         return;
     }
     k_tile_sums<<<ntiles, kScanThreads, 0, s>>>(f.cell_count, P.numc, f.scan_tiles);
-    launch_after(k_cell_scan<false>, ntiles, kScanThreads, s, f.cell_count, P.numc,
-                 f.scan_tiles, f.cell_start, f.occ_list, f.big_list, f.ctr, f.n);
+    if (ntiles <= kScanSumTiles) {
+        scan(k_cell_scan<Before::kSums>);
+    } else {
+        launch_after(k_scan_tiles, 1, 1024, s, f.scan_tiles, ntiles);
+        scan(k_cell_scan<Before::kScanned>);
+    }
 }
 
 void launch_scatter(const Frame &f, const DevParams &P, int max_occ, int num_sms,

@@ -40,10 +40,12 @@ constexpr int kTaskOffsetLimit = 1 << 24;
 constexpr int kMaskRowMax = 32;
 // Scan tile (items per CTA) for the reduce-then-scan kernels.
 constexpr int kScanThreads = 256;
-constexpr int kScanItems = 16;
+constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
-// Up to this many tiles the cell scan needs no tile sums (k_cell_scan).
-constexpr int kScanDirectTiles = 6;
+// Where the cell scan takes what lies before a tile from (k_cell_scan): up to
+// this many tiles from the counts, up to this many from the tiles' sums.
+constexpr int kScanDirectTiles = 12;
+constexpr int kScanSumTiles = 8192;
 // Tiles of the per-occupied-cell {tasks, SMS, TRA} scan of the split.
 constexpr int kValItems = 4;
 constexpr int kValTile = kScanThreads * kValItems;
@@ -138,7 +140,10 @@ struct Counters {
     // compaction is skipped.
     int32_t any_sms;
     int32_t big_fill;       // large cells listed so far by the cell scan
-    int32_t pad[19];
+    // Set by the cell scan when some cell's count could send a cell to the SMS
+    // path; clear, the performance model has nothing to find and is skipped.
+    int32_t crowded;
+    int32_t pad[18];
 };
 
 // Per-frame device pointers of one batch of scenes.

@@ -1402,7 +1402,8 @@ gsph_status gsph_copy_out(gsph_handle h, gsph_field field, void *host_dst,
         case GSPH_FIELD_BLOCK_REQ: {
             int32_t *o = static_cast<int32_t *>(host_dst);
             std::memset(o, 0, size_t(numc) * 4);
-            if (!s.arranged || c.num_occ <= 0) return GSPH_OK;
+            // no cell on the SMS path: no tasks (and no model values kept)
+            if (!s.arranged || c.num_occ <= 0 || !c.any_sms) return GSPH_OK;
             std::vector<int32_t> occ(size_t(c.num_occ));
             std::vector<int4> val(size_t(c.num_occ));
             GSPH_CUDA(cudaMemcpy(occ.data(), s.fr.occ_list, occ.size() * 4,
@@ -1943,7 +1944,7 @@ gsph_status gsph_benchmark(gsph_handle h, int frames, gsph_bench_report *out) {
 size_t gsph_grid_sort_scratch_bytes(uint32_t n, uint32_t numc) {
     const size_t N = std::max<size_t>(n, 1), C = std::max<size_t>(numc, 1);
     const size_t occ = std::max<size_t>(std::min(N, C), 1);
-    const size_t tiles = (C + kScanTile - 1) / kScanTile;
+    const size_t tiles = (C + 4095) / 4096;
     size_t b = 0;
     b += align_up(N * 4, 256);      // key_in
     b += align_up(N * 4, 256);      // slot
@@ -1952,7 +1953,7 @@ size_t gsph_grid_sort_scratch_bytes(uint32_t n, uint32_t numc) {
     b += align_up(C * 4, 256);      // cell_xslab
     b += align_up(occ * 4, 256);    // occ_list
     b += align_up(occ * 4, 256);    // big_list
-    b += align_up(tiles * 8, 256);  // scan tiles
+    b += align_up(tiles * 8, 256);  // reserved: callers keep buffers of this size
     b += align_up(sizeof(Counters), 256);
     return b;
 }
@@ -1992,7 +1993,6 @@ gsph_status gsph_grid_sort_dev(const gsph_params *p, uint32_t n,
     GSPH_CUDA(cudaGetDevice(&dev));
     const size_t N = std::max<size_t>(n, 1), C = size_t(dp.numc);
     const size_t occ = std::max<size_t>(std::min(N, C), 1);
-    const size_t tiles = (C + kScanTile - 1) / kScanTile;
     char *w = static_cast<char *>(scratch);
     auto carve = [&](size_t bytes) {
         char *r = w;
@@ -2023,7 +2023,10 @@ gsph_status gsph_grid_sort_dev(const gsph_params *p, uint32_t n,
     f.cell_count = reinterpret_cast<int32_t *>(carve(C * 4));
     f.ctr = reinterpret_cast<Counters *>(carve(sizeof(Counters)));
     const size_t sum_bytes = size_t(w - sums);
-    f.scan_tiles = reinterpret_cast<unsigned long long *>(carve(tiles * 8));
+    // the scan's tile sums (8 bytes per kScanTile cells) are done with when the
+    // sort writes the slab words
+    f.scan_tiles = reinterpret_cast<unsigned long long *>(f.cell_xslab);
+    static_assert(kScanTile * sizeof(*f.cell_xslab) >= sizeof(*f.scan_tiles), "");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     GSPH_CUDA(cudaMemsetAsync(sums, 0, sum_bytes, s));
     launch_hash_count(f, dp, s);
