@@ -122,6 +122,39 @@ __device__ __forceinline__ MicroPos micro_of(float4 p, const DevParams &P,
     return r;
 }
 
+// A TRA particle's neighbour rows in three registers and the x-y strides: its
+// own cell, and in `flags` which of the nine rows lie in the grid (bits 0-8),
+// whether the left and right cells do (9, 10) and its micro-x slab (11, 12).
+// Eight registers of grid sizes and cell coordinates in the row loop cost a
+// batch 18% of the density pass (5.28M particles in 64 scenes 701 us, with this
+// 627; one scene, whose sizes come as kernel constants, 588 and 596, so it keeps
+// them).
+struct RowFrame {
+    int own, sy, sz;
+    uint32_t flags;
+};
+__device__ __forceinline__ RowFrame row_frame(const MicroPos &mp, const SceneGeom &G) {
+    RowFrame w;
+    w.sy = G.gx;
+    w.sz = G.gx * G.gy;
+    w.own = G.cbase + mp.cx + w.sy * mp.cy + w.sz * mp.cz;
+    const uint32_t y = (mp.cy > 0 ? 1u : 0u) | 2u | (mp.cy + 1 < G.gy ? 4u : 0u);
+    w.flags = (mp.cz > 0 ? y : 0u) | (y << 3) | (mp.cz + 1 < G.gz ? y << 6 : 0u) |
+              (mp.cx > 0 ? 1u << 9 : 0u) | (mp.cx + 1 < G.gx ? 1u << 10 : 0u) |
+              (uint32_t(mp.lmx) << 11);
+    return w;
+}
+__device__ __forceinline__ void tra_row_range(const Frame &f, const RowFrame &w, int m,
+                                              int &begin, int &end) {
+    const int sM = f.cell_start[m];
+    const int eM = f.cell_start[m + 1];
+    const int lmx = int(w.flags >> 11);
+    begin = sM;
+    end = eM;
+    if (w.flags & (1u << 9)) begin = slab_begin(f, m - 1, f.cell_start[m - 1], sM, lmx);
+    if (w.flags & (1u << 10)) end = slab_end(f, m + 1, eM, f.cell_start[m + 2], lmx);
+}
+
 struct ForceAcc {
     float px, py, pz;   // pressure sum
     float vx, vy, vz;   // viscosity sum
@@ -394,7 +427,9 @@ __device__ __forceinline__ int next_unit(int *counter) {
 // L1 rather than DRAM. Chosen on the host when the cell arrays are too large
 // to stay in L2 (large batches); otherwise the extra instructions cost more
 // than they save.
-template <int W, bool kRowPrefetch>
+//
+// kMany: the build for several scenes (RowFrame).
+template <int W, bool kRowPrefetch, bool kMany>
 __global__ void __launch_bounds__(W * 32, 6 * kWarpsPerBlock / W)
 k_density_tra(Frame f, DevParams P) {
     chain_wait();
@@ -430,14 +465,21 @@ k_density_tra(Frame f, DevParams P) {
                 }
             }
         }
+        const RowFrame rows = row_frame(mp, G);   // kMany only
         for (int r = 0; r < 9; ++r) {
             const int ny = mp.cy + (r % 3) - 1;
             const int nz = mp.cz + (r / 3) - 1;
             uint32_t mask = 0u;
-            if (ny >= 0 && ny < G.gy && nz >= 0 && nz < G.gz) {
-                const int m = G.cbase + mp.cx + G.gx * (ny + G.gy * nz);
+            if (kMany ? (rows.flags >> r) & 1u
+                      : ny >= 0 && ny < G.gy && nz >= 0 && nz < G.gz) {
                 int begin, end;
-                row_range(f, G, m, mp.cx, mp.lmx, mp.lmx, begin, end);
+                if constexpr (kMany)
+                    tra_row_range(f, rows,
+                                  rows.own + ((r % 3) - 1) * rows.sy + ((r / 3) - 1) * rows.sz,
+                                  begin, end);
+                else
+                    row_range(f, G, G.cbase + mp.cx + G.gx * (ny + G.gy * nz), mp.cx, mp.lmx,
+                              mp.lmx, begin, end);
                 incomplete |= (end - begin > kMaskRowMax);
                 uint32_t bit = 1u;
 #pragma unroll 8
@@ -1464,10 +1506,9 @@ template <int W>
 cudaError_t configure_shape(int smem) {
     const int k = kWarpsPerBlock / W;   // CTAs per SM scale with the block size
     cudaError_t e;
-    if ((e = set_carveout(k_density_tra<W, false>, kMaxShape.density_tra * k, smem, W * 32)))
-        return e;
-    if ((e = set_carveout(k_density_tra<W, true>, kMaxShape.density_tra * k, smem, W * 32)))
-        return e;
+    for (auto kernel : {k_density_tra<W, false, false>, k_density_tra<W, false, true>,
+                        k_density_tra<W, true, false>, k_density_tra<W, true, true>})
+        if ((e = set_carveout(kernel, kMaxShape.density_tra * k, smem, W * 32))) return e;
     if ((e = set_carveout(k_density_sms<W>, kMaxShape.density_sms * k, smem, W * 32)))
         return e;
     if ((e = set_carveout(k_force_tra<false, W>, kMaxShape.force_tra * k, smem, W * 32)))
@@ -1500,10 +1541,14 @@ void launch_density_w(const Frame &f, const DevParams &P, int num_sms,
         launch_after(k_density_tra_rows<1>, units, 288, s, f, P);
     else if (units <= num_sms * kRowsMax3)
         launch_after(k_density_tra_rows<3>, (units + 2) / 3, 288, s, f, P);
-    else if (row_prefetch)
-        launch_after(k_density_tra<W, true>, num_sms * shape.density_tra, W * 32, s, f, P);
-    else
-        launch_after(k_density_tra<W, false>, num_sms * shape.density_tra, W * 32, s, f, P);
+    else {
+        const bool many = f.scenes.count > 1;
+        launch_after(row_prefetch ? (many ? k_density_tra<W, true, true>
+                                          : k_density_tra<W, true, false>)
+                                  : (many ? k_density_tra<W, false, true>
+                                          : k_density_tra<W, false, false>),
+                     num_sms * shape.density_tra, W * 32, s, f, P);
+    }
 }
 
 template <bool kArt, int W>
