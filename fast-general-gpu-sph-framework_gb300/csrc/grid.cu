@@ -49,7 +49,7 @@ k_hash_count(const float4 *__restrict__ pos, int n, DevParams P, SceneTable T,
     const SceneGeom G = geom_of_particle(T, i);
     const uint32_t key = micro_key(pos[i], P, G, ctr, i);
     key_out[i] = key;
-    slot_out[i] = cell_slot(cell_count, key >> 6, active);
+    slot_out[i] = cell_slot_runs(cell_count, key >> 6, active);
 }
 
 // The particles the split sent to SMS tasks (compact[middle, n)), hashed
@@ -74,7 +74,7 @@ k_hash_sms(const float4 *__restrict__ pos, int n, DevParams P, SceneTable T,
             const SceneGeom G = geom_of_particle(T, i);
             const uint32_t key = micro_key(pos[i], P, G, ctr, i);
             key_out[i] = key;
-            slot_out[i] = cell_slot(cell_count, key >> 6, active);
+            slot_out[i] = cell_slot_runs(cell_count, key >> 6, active);
         }
     }
 }
@@ -487,8 +487,8 @@ __device__ void block_exclusive_scan(const int *in, int *out, int n) {
 // micro cell (counts, scan, scatter) and ranked by value inside their bucket
 // only. Larger cells do the same in global memory with finer buckets. In a
 // frame with SMS cells the block then emits its cell's part of the compact
-// index and its tasks, and the cells of k_sort_small are emitted one per
-// thread (default scene, 3.94M particles: arrange 332 -> 290 us; with a thread
+// index and its tasks, and the cells of k_sort_small are emitted 32 per warp
+// (default scene, 3.94M particles: arrange 332 -> 290 us; with a thread
 // writing all of a 280-particle cell the emission alone took 41 us, and 34 of
 // 64,000 particles' 88).
 __global__ void __launch_bounds__(256) k_sort_big(Frame f) {
@@ -624,15 +624,9 @@ __global__ void __launch_bounds__(256) k_sort_big(Frame f) {
     }
     if (!emit) return;   // all TRA: the compact index is the identity
     const int num_occ = f.ctr->num_occ;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < num_occ;
-         k += gridDim.x * blockDim.x) {
-        const int cell = f.occ_list[k];
-        const int b = f.cell_start[cell];
-        const int n = f.cell_start[cell + 1] - b;
-        if (n <= kSmallCellMax)
-            emit_cell(f, cell, b, n, f.cell_val[k], cells_before(f, k), 0, 1,
-                      [&](int i) { return f.key[b + i]; });
-    }
+    const int warp = int(blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int warps = int(gridDim.x * blockDim.x) >> 5;
+    for (int k0 = warp * 32; k0 < num_occ; k0 += warps * 32) emit_small_cells(f, k0, num_occ);
 }
 
 }  // namespace

@@ -266,13 +266,26 @@ __device__ __forceinline__ uint32_t micro_key(float4 p, const DevParams &P,
     return (c << 6) | sub;
 }
 
-// Slot of a particle among its cell's particles: one atomic per run of
-// consecutive `active` lanes with the same cell. Particles come in the order
-// of the last sort, so a warp holds few runs; match.any, which would also
-// join separate runs of one cell, takes longer the more cells a warp holds
-// (hash of 1.05M particles in no order: 23.5 us against 13.9).
+// Slot of a particle among its cell's particles (lanes in `active`): one
+// atomic per cell per warp, joined by match.any, for the force pass, whose
+// particles are in sorted order and hold few cells per warp (1.2 us less than
+// cell_slot_runs on 3.94M).
 __device__ __forceinline__ uint32_t cell_slot(int32_t *cell_count, uint32_t cell,
                                               unsigned active) {
+    const unsigned peers = __match_any_sync(active, cell);
+    const int lane = threadIdx.x & 31;
+    const int leader = __ffs(peers) - 1;
+    int base = 0;
+    if (lane == leader) base = atomicAdd(&cell_count[cell], __popc(peers));
+    base = __shfl_sync(peers, base, leader);
+    return uint32_t(base + __popc(peers & lanemask_lt()));
+}
+
+// The same with one atomic per run of consecutive lanes with the same cell, for
+// the hash of particles in any order: match.any takes longer the more cells a
+// warp holds (hash of 1.05M particles in no order: 23.5 us against 13.9).
+__device__ __forceinline__ uint32_t cell_slot_runs(int32_t *cell_count, uint32_t cell,
+                                                   unsigned active) {
     const int lane = threadIdx.x & 31;
     const unsigned below = active & lanemask_lt();
     const uint32_t prev = __shfl_sync(active, cell, below ? 31 - __clz(below) : lane);

@@ -191,18 +191,14 @@ __device__ __forceinline__ int4 cells_before(const Frame &f, int k) {
     return add4(f.scan_tiles4[k / kValTile], f.cell_prefix[k]);
 }
 
-// A7/A8: the compact index and the task descriptors of one occupied cell
-// (particles [b, b + n), model values v, pre = cells_before), by `threads`
-// threads numbered `t0`. micro(i) is the micro-cell part of the key of the
-// cell's i-th sorted particle.
+// A8: the task descriptors of one occupied cell (particles [b, b + n), model
+// values v, pre = cells_before), by `threads` threads numbered `t0`. micro(i)
+// is the micro-cell part of the key of the cell's i-th sorted particle.
 template <class Micro>
-__device__ __forceinline__ void emit_cell(const Frame &f, int cell, int b, int n, int4 v,
-                                          int4 pre, int t0, int threads, Micro micro) {
-    const int middle = f.ctr->middle;
-    const int task_count = f.ctr->task_count;
-    for (int j = t0; j < v.z; j += threads) f.compact[pre.z + j] = b + v.y + j;
-    for (int j = t0; j < v.y; j += threads) f.compact[middle + pre.y + j] = b + j;
+__device__ __forceinline__ void emit_tasks(const Frame &f, int cell, int b, int n, int4 v,
+                                           int4 pre, int t0, int threads, Micro micro) {
     if (v.x == 0) return;
+    const int task_count = f.ctr->task_count;
     const SceneGeom G = geom_of_cell(f.scenes, cell);
     const int local = cell - G.cbase;
     const uint16_t cx = uint16_t(local % G.gx);
@@ -252,6 +248,53 @@ __device__ __forceinline__ void emit_cell(const Frame &f, int cell, int b, int n
             pack_bounds(task.xxi, task.xxx, task.yyi, task.yyy, task.zzi, task.zzz);
         f.tasks[ti] = task;
     }
+}
+
+// A7/A8: the compact index and the task descriptors of one occupied cell, by
+// `threads` threads numbered `t0`.
+template <class Micro>
+__device__ __forceinline__ void emit_cell(const Frame &f, int cell, int b, int n, int4 v,
+                                          int4 pre, int t0, int threads, Micro micro) {
+    const int middle = f.ctr->middle;
+    for (int j = t0; j < v.z; j += threads) f.compact[pre.z + j] = b + v.y + j;
+    for (int j = t0; j < v.y; j += threads) f.compact[middle + pre.y + j] = b + j;
+    emit_tasks(f, cell, b, n, v, pre, t0, threads, micro);
+}
+
+// The same for the small cells among 32 occupied cells from k0 on, by a warp:
+// eight lanes write a cell's indices side by side (one thread per cell wrote
+// to 32 sectors at a time: arrange of 3.94M particles with 8 SMS tasks 143.6 ->
+// 140.9 us), a lane its cell's tasks.
+__device__ __forceinline__ void emit_small_cells(const Frame &f, int k0, int num_occ) {
+    const int lane = threadIdx.x & 31;
+    const int k = k0 + lane;
+    int cell = 0, b = 0, n = 0;
+    int4 v = make_int4(0, 0, 0, 0), pre = v;
+    if (k < num_occ) {
+        cell = f.occ_list[k];
+        b = f.cell_start[cell];
+        n = f.cell_start[cell + 1] - b;
+        if (n <= kSmallCellMax) {
+            v = f.cell_val[k];
+            pre = cells_before(f, k);
+        }
+    }
+    const int middle = f.ctr->middle;
+#pragma unroll
+    for (int q = 0; q < 32; q += 4) {
+        const int src = q + (lane >> 3);
+        const int sb = __shfl_sync(0xFFFFFFFFu, b, src);
+        const int sms = __shfl_sync(0xFFFFFFFFu, v.y, src);
+        const int tra = __shfl_sync(0xFFFFFFFFu, v.z, src);
+        const int at = __shfl_sync(0xFFFFFFFFu, pre.z, src);
+        for (int j = lane & 7; j < tra; j += 8) f.compact[at + j] = sb + sms + j;
+        if (__any_sync(0xFFFFFFFFu, sms > 0)) {
+            const int to = middle + __shfl_sync(0xFFFFFFFFu, pre.y, src);
+            for (int j = lane & 7; j < sms; j += 8) f.compact[to + j] = sb + j;
+        }
+    }
+    if (v.x > 0)
+        emit_tasks(f, cell, b, n, v, pre, 0, 1, [&](int i) { return f.key[b + i]; });
 }
 
 }  // namespace
