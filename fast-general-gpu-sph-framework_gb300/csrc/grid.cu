@@ -340,14 +340,42 @@ __device__ __forceinline__ void write_groups(const Frame &f, uint32_t cell,
     dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
 }
 
+// kAll: velocity and evaluated velocity too (else k_gather_motion moves them).
+template <bool kAll>
 __device__ __forceinline__ void move_particle(const Frame &f, int dst,
                                               unsigned long long e) {
     const int src = int(e & 0xFFFFFFFFull);
     f.key[dst] = uint32_t(e >> 32);
     f.perm[dst] = src;
     f.pos[dst] = f.pos_in[src];
-    f.vel[dst] = f.vel_in[src];
-    f.ev[dst] = f.ev_in[src];
+    if (kAll) {
+        f.vel[dst] = f.vel_in[src];
+        f.ev[dst] = f.ev_in[src];
+    }
+}
+
+// Velocity and evaluated velocity after a sort that moved the positions alone;
+// the pressures (ev.w) of a density pass in between stay. Two particles per
+// thread, as k_sort_small.
+__global__ void __launch_bounds__(256) k_gather_motion(Frame f) {
+    const int d0 = blockIdx.x * (2 * blockDim.x) + threadIdx.x;
+    const int d[2] = {d0, d0 + int(blockDim.x)};
+    float4 vel[2], ev[2];
+    float w[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        if (d[k] >= f.n) continue;
+        const int src = f.perm[d[k]];
+        vel[k] = f.vel_in[src];
+        ev[k] = f.ev_in[src];
+        w[k] = f.ev[d[k]].w;
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        if (d[k] >= f.n) continue;
+        f.vel[d[k]] = vel[k];
+        f.ev[d[k]] = make_float4(ev[k].x, ev[k].y, ev[k].z, w[k]);
+    }
 }
 
 // Group offsets and slab words of a small cell, written by the thread of the
@@ -380,6 +408,7 @@ __device__ __forceinline__ void small_cell_groups(const Frame &f, uint32_t cell,
 // that the two chains of loads are in flight together.
 // Where a split is made, the first block scans the performance model's tile
 // sums instead.
+template <bool kAll>
 __global__ void __launch_bounds__(256) k_sort_small(Frame f) {
     chain_wait();
     chain_next();
@@ -415,8 +444,10 @@ __global__ void __launch_bounds__(256) k_sort_small(Frame f) {
         if (live[k]) {
             const int src = int(e[k] & 0xFFFFFFFFull);
             pos[k] = f.pos_in[src];
-            vel[k] = f.vel_in[src];
-            ev[k] = f.ev_in[src];
+            if (kAll) {
+                vel[k] = f.vel_in[src];
+                ev[k] = f.ev_in[src];
+            }
         }
     }
 #pragma unroll
@@ -430,8 +461,10 @@ __global__ void __launch_bounds__(256) k_sort_small(Frame f) {
         f.key[dst] = uint32_t(e[k] >> 32);
         f.perm[dst] = int(e[k] & 0xFFFFFFFFull);
         f.pos[dst] = pos[k];
-        f.vel[dst] = vel[k];
-        f.ev[dst] = ev[k];
+        if (kAll) {
+            f.vel[dst] = vel[k];
+            f.ev[dst] = ev[k];
+        }
         if (rank[k] == 0) small_cell_groups(f, uint32_t(e[k] >> 38), b[k], cnt[k]);
     }
 }
@@ -491,6 +524,7 @@ __device__ void block_exclusive_scan(const int *in, int *out, int n) {
 // (default scene, 3.94M particles: arrange 332 -> 290 us; with a thread
 // writing all of a 280-particle cell the emission alone took 41 us, and 34 of
 // 64,000 particles' 88).
+template <bool kAll>
 __global__ void __launch_bounds__(256) k_sort_big(Frame f) {
     __shared__ unsigned long long sp[kBigCellSmem];
     __shared__ uint16_t order[kBigCellSmem];
@@ -547,7 +581,7 @@ __global__ void __launch_bounds__(256) k_sort_big(Frame f) {
                 int rank = mstart[m];
                 for (int k = mstart[m]; k < mstart[m + 1]; ++k)
                     rank += (sp[order[k]] < e) ? 1 : 0;
-                move_particle(f, b + rank, e);
+                move_particle<kAll>(f, b + rank, e);
             }
             if (threadIdx.x == 0) {
                 int n16[16];
@@ -606,7 +640,7 @@ __global__ void __launch_bounds__(256) k_sort_big(Frame f) {
             int rank = bstart[k];
             for (int q = bstart[k]; q < bstart[k + 1]; ++q)
                 rank += (src[order_g[q]] < e) ? 1 : 0;
-            move_particle(f, b + rank, e);
+            move_particle<kAll>(f, b + rank, e);
             atomicAdd(&grp[int((e >> 34) & 15ull)], 1);
         }
         __syncthreads();
@@ -682,10 +716,16 @@ void launch_scatter(const Frame &f, const DevParams &P, int max_occ, int num_sms
                  kScanThreads, s, f, P, model);
 }
 
-void launch_cell_sort(const Frame &f, int num_sms, cudaStream_t s) {
+void launch_cell_sort(const Frame &f, int num_sms, cudaStream_t s, bool motion) {
     if (f.n <= 0) return;
-    launch_after(k_sort_small, (f.n + 511) / 512 + (f.cell_val ? 1 : 0), 256, s, f);
-    launch_after(k_sort_big, num_sms * 4, 256, s, f);
+    launch_after(motion ? k_sort_small<true> : k_sort_small<false>,
+                 (f.n + 511) / 512 + (f.cell_val ? 1 : 0), 256, s, f);
+    launch_after(motion ? k_sort_big<true> : k_sort_big<false>, num_sms * 4, 256, s, f);
+}
+
+void launch_gather_motion(const Frame &f, cudaStream_t s) {
+    if (f.n <= 0) return;
+    k_gather_motion<<<(f.n + 511) / 512, 256, 0, s>>>(f);
 }
 
 }  // namespace gsph

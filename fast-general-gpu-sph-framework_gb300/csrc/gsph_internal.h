@@ -316,7 +316,10 @@ void launch_scatter(const Frame &f, const DevParams &P, int max_occ, int num_sms
                     cudaStream_t s);
 // The order inside the cells and, where f.cell_val is set, the TRA/SMS
 // partition and the SMS tasks; launch_judge then pairs the tasks (judgeTask).
-void launch_cell_sort(const Frame &f, int num_sms, cudaStream_t s);
+// motion: velocity and evaluated velocity are sorted with the position;
+// without, launch_gather_motion does it later, from pos_in's order to pos's.
+void launch_cell_sort(const Frame &f, int num_sms, cudaStream_t s, bool motion = true);
+void launch_gather_motion(const Frame &f, cudaStream_t s);
 // ---- launchers (split.cu) ----
 void launch_judge(const Frame &f, int max_occ, int num_sms, cudaStream_t s);
 // ---- launchers (physics.cu) ----

@@ -128,6 +128,10 @@ struct System {
     cudaEvent_t xfer_done[3] = {nullptr, nullptr, nullptr};
     cudaEvent_t frames_done = nullptr;
     bool xfer_pending = false;
+    // The upload of the velocities runs on a third stream, behind that of the
+    // positions, and is waited for only where the first frame needs them.
+    cudaStream_t upload = nullptr;
+    cudaEvent_t pos_up = nullptr, motion_up = nullptr;
 
     void join_xfer() {
         if (!xfer_pending) return;
@@ -177,10 +181,16 @@ struct System {
                 cudaEventDestroy(e);
                 e = nullptr;
             }
-        if (frames_done) {
-            cudaEventDestroy(frames_done);
-            frames_done = nullptr;
+        if (upload) {
+            cudaStreamSynchronize(upload);
+            cudaStreamDestroy(upload);
+            upload = nullptr;
         }
+        for (cudaEvent_t *e : {&frames_done, &pos_up, &motion_up})
+            if (*e) {
+                cudaEventDestroy(*e);
+                *e = nullptr;
+            }
         if (aux) {
             cudaStreamSynchronize(aux);
             cudaStreamDestroy(aux);
@@ -546,14 +556,15 @@ struct System {
     }
 
     // pair_tasks: also pair the SMS tasks (judgeTask) here; a frame leaves
-    // that to its density stage, on the second stream.
-    void enqueue_arrange(int in, bool pair_tasks = true) {
+    // that to its density stage, on the second stream. motion: see
+    // launch_cell_sort.
+    void enqueue_arrange(int in, bool pair_tasks = true, bool motion = true) {
         lists_valid = false;
         const Frame f = frame_arrange(in);
         if (!hashed) enqueue_hash(in);
         launch_cell_scan(f, dp, stream);
         launch_scatter(f, dp, max_occ, num_sms, stream);
-        launch_cell_sort(f, num_sms, stream);
+        launch_cell_sort(f, num_sms, stream, motion);
         if (pair_tasks) launch_judge(f, max_occ, num_sms, stream);
         hashed = false;          // consumed; the sort cleared the counts
         counts_dirty = false;
@@ -680,6 +691,24 @@ struct System {
         gsph_status st = check_launch();
         if (st) return st;
         cur = in;
+        arranged = true;
+        grid_current = false;
+        ++frames;
+        return GSPH_OK;
+    }
+
+    // The first frame of gsph_step_host_async, as tick(): the velocities are
+    // still on their way while the positions are sorted and the density pass,
+    // which needs only them, runs (motion_up: the upload's end).
+    gsph_status tick_uploading(bool keep_acc) {
+        const int in = cur, out = 1 - cur;
+        enqueue_arrange(in, false, false);
+        enqueue_density(out, true);
+        GSPH_CUDA(cudaStreamWaitEvent(stream, motion_up, 0));
+        launch_gather_motion(frame_arrange(in), stream);
+        enqueue_force_advance(out, keep_acc);
+        gsph_status st = check_launch();
+        if (st) return st;
         arranged = true;
         grid_current = false;
         ++frames;
@@ -1592,25 +1621,42 @@ gsph_status gsph_step_host_async(gsph_handle h, int frames, void *pos4, void *ve
     }
     if (!s.xfer) {
         GSPH_CUDA(cudaStreamCreateWithFlags(&s.xfer, cudaStreamNonBlocking));
+        GSPH_CUDA(cudaStreamCreateWithFlags(&s.upload, cudaStreamNonBlocking));
         for (auto &e : s.xfer_done)
             GSPH_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        GSPH_CUDA(cudaEventCreateWithFlags(&s.frames_done, cudaEventDisableTiming));
+        for (cudaEvent_t *e : {&s.frames_done, &s.pos_up, &s.motion_up})
+            GSPH_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     }
     const gsph_field fields[3] = {GSPH_FIELD_POSITION, GSPH_FIELD_VELOCITY,
                                   GSPH_FIELD_EVAL_VELOCITY};
     void *host[3] = {pos4, vel4, ev4};
     const size_t bytes = size_t(s.n) * sizeof(float4);
-    // upload: each array after its previous return copy (if any) is done
+    // upload: each array after its previous return copy (if any) is done; the
+    // velocities behind the positions, beside the first frame's work on these
     for (int k = 0; k < 3; ++k) {
-        if (s.xfer_pending) GSPH_CUDA(cudaStreamWaitEvent(s.stream, s.xfer_done[k], 0));
+        cudaStream_t up = k == 0 ? s.stream : s.upload;
+        if (s.xfer_pending) GSPH_CUDA(cudaStreamWaitEvent(up, s.xfer_done[k], 0));
         if (bytes)
             GSPH_CUDA(cudaMemcpyAsync(state_ptr(s, fields[k]), host[k], bytes,
-                                      cudaMemcpyHostToDevice, s.stream));
+                                      cudaMemcpyHostToDevice, up));
+        if (k == 0) {
+            GSPH_CUDA(cudaEventRecord(s.pos_up, s.stream));
+            GSPH_CUDA(cudaStreamWaitEvent(s.upload, s.pos_up, 0));
+        }
     }
+    GSPH_CUDA(cudaEventRecord(s.motion_up, s.upload));
     s.xfer_pending = false;
     s.lists_valid = false;
     s.grid_current = false;
     s.hashed = false;
+    // a first frame launched kernel by kernel overlaps the velocities' upload
+    const bool graphs = s.graph_frames > 0 && frames >= s.graph_frames;
+    if (frames > 0 && bytes && !graphs && !s.timing) {
+        if ((st = s.tick_uploading(frames == 1))) return st;
+        --frames;
+    } else {
+        GSPH_CUDA(cudaStreamWaitEvent(s.stream, s.motion_up, 0));
+    }
     if ((st = s.step(frames))) return st;
     if ((st = s.check_launch())) return st;
     // return copies on the transfer stream, after the frames
