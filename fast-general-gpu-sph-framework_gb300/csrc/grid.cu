@@ -265,6 +265,8 @@ k_cell_scan(const int32_t *__restrict__ count, int numc,
         ctr->work_force = 0;
         ctr->work_density_sms = 0;
         ctr->work_force_sms = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) ctr->work_force_part[k] = 0;
         // all TRA, unless the performance model finds an SMS cell
         ctr->any_sms = 0;
         ctr->task_count = 0;

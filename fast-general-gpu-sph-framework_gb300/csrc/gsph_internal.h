@@ -143,7 +143,8 @@ struct Counters {
     // Set by the cell scan when some cell's count could send a cell to the SMS
     // path; clear, the performance model has nothing to find and is skipped.
     int32_t crowded;
-    int32_t pad[18];
+    int32_t work_force_part[4];   // work counters of a force pass in parts
+    int32_t pad[14];
 };
 
 // Per-frame device pointers of one batch of scenes.
@@ -341,6 +342,18 @@ void launch_density(const Frame &f, const DevParams &P, int num_sms,
 // masks are valid.
 void launch_force(const Frame &f, const DevParams &P, int num_sms, bool fresh,
                   const LaunchShape &shape, cudaStream_t s, cudaStream_t s_sms);
+// Its two sides by themselves, and a part of the TRA side: the particles
+// [32 begin, 32 end) of the compact index, so that all TRA particles among the
+// first 32 end sorted ones are done after the parts up to it. Parts (at most 4,
+// `queue` their number) suit scenes past the small-scene builds.
+struct ForcePart {
+    int begin, end, queue;
+};
+bool force_in_parts(const Frame &f, int num_sms);
+void launch_force_sms(const Frame &f, const DevParams &P, int num_sms,
+                      const LaunchShape &shape, cudaStream_t s);
+void launch_force_tra_part(const Frame &f, const DevParams &P, int num_sms, bool fresh,
+                           const LaunchShape &shape, const ForcePart &part, cudaStream_t s);
 void launch_integrate(const Frame &f, const DevParams &P, cudaStream_t s);
 // Render-side buffers (headless): packed RGBA colour per particle from its
 // density and its path (TRA, paired SMS, single SMS), and render-space

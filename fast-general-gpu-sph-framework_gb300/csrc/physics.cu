@@ -25,6 +25,7 @@
 // sorted index; the TRA density pass records which interact as bit masks that
 // the TRA force pass walks.
 #include <algorithm>
+#include <type_traits>
 
 #include "gsph_internal.h"
 
@@ -947,9 +948,11 @@ __device__ __forceinline__ void force_scan(const Frame &f, const DevParams &P,
 // warps taking turns on one counter cost more than the work), and four
 // neighbours' loads instead of two are in flight before the first of them is
 // evaluated (the order of the sums is unchanged).
-template <bool kArt, int W, bool kSmall = false>
+//
+// kPart: only the units of `part`.
+template <bool kArt, int W, bool kSmall = false, bool kPart = false>
 __global__ void __launch_bounds__(W * 32, kSmall ? 1 : 4 * kWarpsPerBlock / W)
-k_force_tra(Frame f, DevParams P, bool fresh) {
+k_force_tra(Frame f, DevParams P, bool fresh, ForcePart part) {
     __shared__ uint32_t row_mask[9][W * 32];
     __shared__ int row_start[9][W * 32];
     const int lane = threadIdx.x & 31;
@@ -959,9 +962,10 @@ k_force_tra(Frame f, DevParams P, bool fresh) {
     if (units == 0) return;        // no TRA work: skip the queue atomics
     for (bool first = true;; first = false) {
         if (kSmall && !first) break;
-        const int u = kSmall ? int(blockIdx.x * W + (threadIdx.x >> 5))
-                             : next_unit(&f.ctr->work_force);
-        if (u >= units) break;
+        const int u = kSmall  ? int(blockIdx.x * W + (threadIdx.x >> 5))
+                      : kPart ? part.begin + next_unit(&f.ctr->work_force_part[part.queue])
+                              : next_unit(&f.ctr->work_force);
+        if (u >= (kPart ? min(units, part.end) : units)) break;
         const int idx = (u << 5) + lane;
         if (idx >= middle) continue;
         const int self = ident ? idx : f.compact[idx];
@@ -1511,10 +1515,9 @@ cudaError_t configure_shape(int smem) {
         if ((e = set_carveout(kernel, kMaxShape.density_tra * k, smem, W * 32))) return e;
     if ((e = set_carveout(k_density_sms<W>, kMaxShape.density_sms * k, smem, W * 32)))
         return e;
-    if ((e = set_carveout(k_force_tra<false, W>, kMaxShape.force_tra * k, smem, W * 32)))
-        return e;
-    if ((e = set_carveout(k_force_tra<true, W>, kMaxShape.force_tra * k, smem, W * 32)))
-        return e;
+    for (auto kernel : {k_force_tra<false, W>, k_force_tra<true, W>,
+                        k_force_tra<false, W, false, true>, k_force_tra<true, W, false, true>})
+        if ((e = set_carveout(kernel, kMaxShape.force_tra * k, smem, W * 32))) return e;
     if ((e = set_carveout(k_force_sms<false, W>, kForceSmsCtas * k, smem, W * 32)))
         return e;
     return set_carveout(k_force_sms<true, W>, kForceSmsCtas * k, smem, W * 32);
@@ -1552,17 +1555,39 @@ void launch_density_w(const Frame &f, const DevParams &P, int num_sms,
 }
 
 template <bool kArt, int W>
-void launch_force_w(const Frame &f, const DevParams &P, int num_sms, bool fresh,
-                    const LaunchShape &shape, cudaStream_t s, cudaStream_t s_sms) {
-    k_force_sms<kArt, W><<<sms_blocks(f, num_sms, shape.force_sms, W), W * 32, 0, s_sms>>>(
+void launch_force_sms_w(const Frame &f, const DevParams &P, int num_sms,
+                        const LaunchShape &shape, cudaStream_t s) {
+    k_force_sms<kArt, W><<<sms_blocks(f, num_sms, shape.force_sms, W), W * 32, 0, s>>>(
         f, P, num_sms * kForceSmsCtas * kWarpsPerBlock / W);
+}
+
+// part: null for all units.
+template <bool kArt, int W>
+void launch_force_tra_w(const Frame &f, const DevParams &P, int num_sms, bool fresh,
+                        const LaunchShape &shape, const ForcePart *part, cudaStream_t s) {
     const int units = (f.n + 31) / 32;
-    if (units <= num_sms * kForceQuadMax)
+    if (part)
+        k_force_tra<kArt, W, false, true>
+            <<<num_sms * shape.force_tra, W * 32, 0, s>>>(f, P, fresh, *part);
+    else if (units <= num_sms * kForceQuadMax)
         k_force_tra_quad<kArt><<<units, 128, 0, s>>>(f, P, fresh);
     else if (units <= num_sms * kForceSmallMax)
-        k_force_tra<kArt, 2, true><<<(units + 1) / 2, 64, 0, s>>>(f, P, fresh);
+        k_force_tra<kArt, 2, true><<<(units + 1) / 2, 64, 0, s>>>(f, P, fresh, ForcePart{});
     else
-        k_force_tra<kArt, W><<<num_sms * shape.force_tra, W * 32, 0, s>>>(f, P, fresh);
+        k_force_tra<kArt, W>
+            <<<num_sms * shape.force_tra, W * 32, 0, s>>>(f, P, fresh, ForcePart{});
+}
+
+// Calls run(viscosity model, block shape) with both as compile-time constants.
+template <class Run>
+void with_build(const DevParams &P, const LaunchShape &shape, Run run) {
+    using Full = std::integral_constant<int, kWarpsPerBlock>;
+    using Half = std::integral_constant<int, kWarpsPerBlock / 2>;
+    const bool half = shape.warps == kWarpsPerBlock / 2;
+    if (P.visc_artificial)
+        half ? run(std::true_type{}, Half{}) : run(std::true_type{}, Full{});
+    else
+        half ? run(std::false_type{}, Half{}) : run(std::false_type{}, Full{});
 }
 
 }  // namespace
@@ -1587,21 +1612,33 @@ void launch_density(const Frame &f, const DevParams &P, int num_sms,
         launch_density_w<kWarpsPerBlock>(f, P, num_sms, shape, s, s_sms, row_prefetch);
 }
 
+bool force_in_parts(const Frame &f, int num_sms) {
+    return (f.n + 31) / 32 > num_sms * kForceSmallMax;
+}
+
+void launch_force_sms(const Frame &f, const DevParams &P, int num_sms,
+                      const LaunchShape &shape, cudaStream_t s) {
+    if (f.n <= 0) return;
+    with_build(P, shape, [&](auto art, auto warps) {
+        launch_force_sms_w<art.value, warps.value>(f, P, num_sms, shape, s);
+    });
+}
+
+void launch_force_tra_part(const Frame &f, const DevParams &P, int num_sms, bool fresh,
+                           const LaunchShape &shape, const ForcePart &part, cudaStream_t s) {
+    if (f.n <= 0) return;
+    with_build(P, shape, [&](auto art, auto warps) {
+        launch_force_tra_w<art.value, warps.value>(f, P, num_sms, fresh, shape, &part, s);
+    });
+}
+
 void launch_force(const Frame &f, const DevParams &P, int num_sms, bool fresh,
                   const LaunchShape &shape, cudaStream_t s, cudaStream_t s_sms) {
     if (f.n <= 0) return;
-    const bool half = shape.warps == kWarpsPerBlock / 2;
-    if (P.visc_artificial) {
-        if (half)
-            launch_force_w<true, kWarpsPerBlock / 2>(f, P, num_sms, fresh, shape, s, s_sms);
-        else
-            launch_force_w<true, kWarpsPerBlock>(f, P, num_sms, fresh, shape, s, s_sms);
-    } else {
-        if (half)
-            launch_force_w<false, kWarpsPerBlock / 2>(f, P, num_sms, fresh, shape, s, s_sms);
-        else
-            launch_force_w<false, kWarpsPerBlock>(f, P, num_sms, fresh, shape, s, s_sms);
-    }
+    launch_force_sms(f, P, num_sms, shape, s_sms);
+    with_build(P, shape, [&](auto art, auto warps) {
+        launch_force_tra_w<art.value, warps.value>(f, P, num_sms, fresh, shape, nullptr, s);
+    });
 }
 
 void launch_integrate(const Frame &f, const DevParams &P, cudaStream_t s) {

@@ -587,13 +587,17 @@ struct System {
     // buffer 1 - b (the previous frame's unsorted copy, no longer read), in
     // buffer b's order. keep_acc: also store the acceleration (the last frame
     // of a step does, so GSPH_FIELD_ACCELERATION holds it afterwards).
-    void enqueue_force_advance(int b, bool keep_acc = true) {
+    Frame frame_force_advance(int b, bool keep_acc) const {
         Frame f = frame_physics(b);
         if (!keep_acc) f.acc = nullptr;
         f.pos_next = pos[1 - b];
         f.vel_next = vel[1 - b];
         f.ev_next = ev[1 - b];
         f.hash_next = true;
+        return f;
+    }
+    void enqueue_force_advance(int b, bool keep_acc = true) {
+        const Frame f = frame_force_advance(b, keep_acc);
         fork();
         launch_force(f, dp, num_sms, lists_valid, shape, stream, aux);
         // the SMS particles' keys ahead, after their force pass on the
@@ -697,17 +701,72 @@ struct System {
         return GSPH_OK;
     }
 
-    // The first frame of gsph_step_host_async, as tick(): the velocities are
-    // still on their way while the positions are sorted and the density pass,
-    // which needs only them, runs (motion_up: the upload's end).
-    gsph_status tick_uploading(bool keep_acc) {
+    // enqueue_force_advance of a last frame whose state goes back to host
+    // memory: the TRA side in parts of 1/8, 2/8 and 5/8 of the particles, and
+    // each part's rows on their way back while the next ones are computed.
+    // The link takes about twice the pass's time, so the first part is what it
+    // waits for, and every part costs a tail: 3.94M particles, calls back to
+    // back, 1,776 us with these parts, 1,859 with 1/8 + 3/8 + 1/2, 1,840 with
+    // 1/16 + 3/16 + 3/4, 1,965 with 1/4 + 3/8 + 3/8, 1,940 in one piece; 1.05M, one
+    // call at a time, 764 -> 684 us. Scenes of the small-scene builds go back
+    // whole.
+    gsph_status force_downloading(int b, bool keep_acc, void *const host[3]) {
+        const Frame f = frame_force_advance(b, keep_acc);
+        const bool split = force_in_parts(f, num_sms);
+        const int units = (n + 31) / 32;
+        const int ends[4] = {0, units / 8, units / 8 * 3, units};
+        const float4 *src[3] = {f.pos_next, f.vel_next, f.ev_next};
+        fork();
+        if (split) {
+            launch_force_sms(f, dp, num_sms, shape, aux);
+        } else {
+            launch_force(f, dp, num_sms, lists_valid, shape, stream, aux);
+        }
+        launch_hash_sms(f, f.pos_next, dp, aux);
+        GSPH_CUDA(cudaEventRecord(join_ev, aux));
+        GSPH_CUDA(cudaStreamWaitEvent(xfer, join_ev, 0));   // the SMS rows, anywhere
+        for (int q = split ? 0 : 2; q < 3; ++q) {
+            const int first = split ? ends[q] : 0, last = ends[q + 1];
+            if (split)
+                launch_force_tra_part(f, dp, num_sms, lists_valid, shape,
+                                      ForcePart{first, last, q}, stream);
+            GSPH_CUDA(cudaEventRecord(frames_done, stream));
+            GSPH_CUDA(cudaStreamWaitEvent(xfer, frames_done, 0));
+            const size_t row = size_t(first) * 32;
+            const size_t rows = std::min(size_t(last) * 32, size_t(n)) - row;
+            for (int k = 0; k < 3; ++k) {
+                GSPH_CUDA(cudaMemcpyAsync(static_cast<float4 *>(host[k]) + row, src[k] + row,
+                                          sizeof(float4) * rows, cudaMemcpyDeviceToHost, xfer));
+                if (q == 2) GSPH_CUDA(cudaEventRecord(xfer_done[k], xfer));
+            }
+        }
+        GSPH_CUDA(cudaStreamWaitEvent(stream, join_ev, 0));
+        lists_valid = false;
+        hashed = true;
+        counts_dirty = true;
+        xfer_pending = true;
+        return GSPH_OK;
+    }
+
+    // A frame of gsph_step_host_async, as tick(). first: the velocities are
+    // still on their way (motion_up: the upload's end) while the positions are
+    // sorted and the density pass, which needs only them, runs (1.05M particles:
+    // 917 -> 764 us a call; the gather that this adds reads and writes each
+    // velocity once). last: the state goes back to `host`.
+    gsph_status tick_host(bool first, bool last, void *const host[3]) {
         const int in = cur, out = 1 - cur;
-        enqueue_arrange(in, false, false);
+        enqueue_arrange(in, false, !first);
         enqueue_density(out, true);
-        GSPH_CUDA(cudaStreamWaitEvent(stream, motion_up, 0));
-        launch_gather_motion(frame_arrange(in), stream);
-        enqueue_force_advance(out, keep_acc);
-        gsph_status st = check_launch();
+        if (first) {
+            GSPH_CUDA(cudaStreamWaitEvent(stream, motion_up, 0));
+            launch_gather_motion(frame_arrange(in), stream);
+        }
+        gsph_status st = GSPH_OK;
+        if (last)
+            st = force_downloading(out, true, host);
+        else
+            enqueue_force_advance(out, false);
+        if (!st) st = check_launch();
         if (st) return st;
         arranged = true;
         grid_current = false;
@@ -1649,14 +1708,16 @@ gsph_status gsph_step_host_async(gsph_handle h, int frames, void *pos4, void *ve
     s.lists_valid = false;
     s.grid_current = false;
     s.hashed = false;
-    // a first frame launched kernel by kernel overlaps the velocities' upload
+    // frames launched kernel by kernel overlap the copies with the first and
+    // the last of them
     const bool graphs = s.graph_frames > 0 && frames >= s.graph_frames;
     if (frames > 0 && bytes && !graphs && !s.timing) {
-        if ((st = s.tick_uploading(frames == 1))) return st;
-        --frames;
-    } else {
-        GSPH_CUDA(cudaStreamWaitEvent(s.stream, s.motion_up, 0));
+        if ((st = s.tick_host(true, frames == 1, host))) return st;
+        for (int k = 1; k < frames; ++k)
+            if ((st = s.tick_host(false, k == frames - 1, host))) return st;
+        return GSPH_OK;
     }
+    GSPH_CUDA(cudaStreamWaitEvent(s.stream, s.motion_up, 0));
     if ((st = s.step(frames))) return st;
     if ((st = s.check_launch())) return st;
     // return copies on the transfer stream, after the frames

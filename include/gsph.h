@@ -362,10 +362,11 @@ gsph_status gsph_copy_out_async(gsph_handle h, gsph_field field,
  * velocity (float4[N] each, the handle's current order, pinned memory) from
  * the three arrays, runs `frames` frames and downloads the new state into the
  * same arrays (HybridSystem::tick with the state kept on the host). Asynchronous:
- * the arrays are complete after gsph_sync. The downloads run on an internal
- * stream, so the upload of an array by the next call waits only for that
- * array's own download (the three round trips overlap); every other call on
- * the handle first waits for all of them. */
+ * the arrays are complete after gsph_sync. Both ways run on internal streams:
+ * the velocities go up beside the first frame's sort and density pass, the state
+ * of a large scene goes back in parts while the last force pass still runs, and
+ * the next call's upload of an array waits only for that array's own download;
+ * every other call on the handle first waits for all of them. */
 gsph_status gsph_step_host_async(gsph_handle h, int frames, void *pos4, void *vel4,
                                  void *ev4);
 

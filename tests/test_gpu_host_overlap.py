@@ -1,6 +1,7 @@
 """gsph_step_host_async overlaps its copies with the first and last frame's
 passes (velocities go up while the positions are sorted and the density pass
-runs). Its results are those of frames on resident state, bit for bit, for
+runs; past the small-scene builds the state goes back in parts of the force
+pass). Its results are those of frames on resident state, bit for bit, for
 every way the frames are launched, for scenes with small cells, cells of the
 block-level sort, both paths side by side, and sizes that divide by nothing."""
 import numpy as np
@@ -11,11 +12,11 @@ from gpu_helpers import dam_scene, dense_scene, shuffled
 pytestmark = pytest.mark.gpu
 
 
-def mixed(gsph):
+def mixed(gsph, n_side=18, loose=3001):
     """A dense block (SMS, cells past 32 particles) in a sparse cloud (TRA)."""
-    _, p, dense = dense_scene(gsph, n_side=18)
+    _, p, dense = dense_scene(gsph, n_side=n_side)
     rng = np.random.default_rng(3)
-    cloud = np.zeros((3001, 4), np.float32)
+    cloud = np.zeros((loose, 4), np.float32)
     cloud[:, :3] = rng.uniform(0.2, 0.4, (len(cloud), 3))
     return None, p, np.concatenate([dense, cloud])
 
@@ -25,6 +26,7 @@ SCENES = {
     "odd": lambda g: (None, *[dam_scene(g, n_side=13)[k] for k in (1, 2)]),
     "past the small builds": lambda g: dam_scene(g, n_side=52, box=(1.2, 1.2, 1.2)),
     "mixed": mixed,
+    "mixed, in parts": lambda g: mixed(g, n_side=52, loose=9001),
 }
 
 
