@@ -841,7 +841,8 @@ __device__ __forceinline__ void cluster_stream(const Frame &f, const SceneGeom &
 
 // ------------------------------------------------------------ density SMS --
 // One cluster of kDenCluster particles per warp (density_kernels.cu:368-565).
-// Bound by issue slots, more than half of them in the candidate tests.
+// Bound by issue slots, about two fifths of them in the candidate tests
+// and the staging.
 // Candidates are staged as pairs (slots 2k, 2k+1), an (x, x, y, y) float4 and
 // a (z, z) float2, and evaluated two at a time with packed FP32x2 arithmetic
 // and the TRA pass's one-compare cut-off test; the groups' sums are added at
