@@ -342,14 +342,18 @@ void launch_density(const Frame &f, const DevParams &P, int num_sms,
 // masks are valid.
 void launch_force(const Frame &f, const DevParams &P, int num_sms, bool fresh,
                   const LaunchShape &shape, cudaStream_t s, cudaStream_t s_sms);
-// Its two sides by themselves, and a part of the TRA side: the particles
+// Whether the TRA passes' blocks fill the GPU for long: an SMS kernel that comes
+// later than they do runs after them, so there the SMS side has to be first in
+// line, and the TRA density pass may not be scheduled ahead of it.
+bool tra_fills(const Frame &f, int num_sms);
+bool force_in_parts(const Frame &f, int num_sms);
+// The force pass's two sides by themselves, and a part of the TRA side: the particles
 // [32 begin, 32 end) of the compact index, so that all TRA particles among the
 // first 32 end sorted ones are done after the parts up to it. Parts (at most 4,
 // `queue` their number) suit scenes past the small-scene builds.
 struct ForcePart {
     int begin, end, queue;
 };
-bool force_in_parts(const Frame &f, int num_sms);
 void launch_force_sms(const Frame &f, const DevParams &P, int num_sms,
                       const LaunchShape &shape, cudaStream_t s);
 void launch_force_tra_part(const Frame &f, const DevParams &P, int num_sms, bool fresh,

@@ -403,6 +403,12 @@ constexpr int kRowsMax1 = 5;
 constexpr int kRowsMax3 = 17;
 constexpr int kForceQuadMax = 5;
 constexpr int kForceSmallMax = 27;
+// From how many units per SM the SMS side is put first in line (tra_fills).
+// Frame times in graphs with the TRA side first / the SMS side first, us, no SMS
+// work: 110,592 particles (23) 78.5 / 83.7, 262,144 (54) 108.0 / 109.2, 373,248
+// (77) 134.8 / 135.4, 1M (206) 297.4 / 296.9, 3.94M (811) 1,047 / 1,043; 3.94M with
+// 8 SMS tasks 1,214 / 1,203.
+constexpr int kTraFills = 128;
 
 // Warps per block of the density and force kernels: 8 by default; each
 // kernel is also built for 4 (gsph_tuning.warps_per_block), with twice the
@@ -1547,11 +1553,14 @@ void launch_density_w(const Frame &f, const DevParams &P, int num_sms,
         launch_after(k_density_tra_rows<3>, (units + 2) / 3, 288, s, f, P);
     else {
         const bool many = f.scenes.count > 1;
-        launch_after(row_prefetch ? (many ? k_density_tra<W, true, true>
-                                          : k_density_tra<W, true, false>)
-                                  : (many ? k_density_tra<W, false, true>
-                                          : k_density_tra<W, false, false>),
-                     num_sms * shape.density_tra, W * 32, s, f, P);
+        auto kernel = row_prefetch ? (many ? k_density_tra<W, true, true>
+                                           : k_density_tra<W, true, false>)
+                                   : (many ? k_density_tra<W, false, true>
+                                           : k_density_tra<W, false, false>);
+        if (tra_fills(f, num_sms))
+            kernel<<<num_sms * shape.density_tra, W * 32, 0, s>>>(f, P);
+        else
+            launch_after(kernel, num_sms * shape.density_tra, W * 32, s, f, P);
     }
 }
 
@@ -1613,6 +1622,9 @@ void launch_density(const Frame &f, const DevParams &P, int num_sms,
         launch_density_w<kWarpsPerBlock>(f, P, num_sms, shape, s, s_sms, row_prefetch);
 }
 
+bool tra_fills(const Frame &f, int num_sms) {
+    return (f.n + 31) / 32 > num_sms * kTraFills;
+}
 bool force_in_parts(const Frame &f, int num_sms) {
     return (f.n + 31) / 32 > num_sms * kForceSmallMax;
 }

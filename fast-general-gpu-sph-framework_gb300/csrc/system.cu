@@ -131,7 +131,7 @@ struct System {
     // The upload of the velocities runs on a third stream, behind that of the
     // positions, and is waited for only where the first frame needs them.
     cudaStream_t upload = nullptr;
-    cudaEvent_t pos_up = nullptr, motion_up = nullptr;
+    cudaEvent_t pos_up = nullptr, motion_up = nullptr, sms_done = nullptr;
 
     void join_xfer() {
         if (!xfer_pending) return;
@@ -140,12 +140,19 @@ struct System {
     }
     std::vector<std::vector<cudaEvent_t>> ev_pending;   // 5 events per frame
 
-    // The SMS side of the density and force stages (task pairing, SMS
-    // density, SMS force) runs on a second stream beside the TRA passes:
-    // fork() orders it after the main stream's work so far, join() orders
-    // the main stream after it. Inside a capture the pair becomes a fork
-    // and a join of the graph. In an all-TRA frame the SMS launches, which
-    // find no work, then cost the frame nothing.
+    // The TRA and the SMS side (SMS density and force, task pairing, look-ahead
+    // hash) of the density and force stages run on two streams: fork() orders
+    // the second one after the main stream's work so far, join() orders the
+    // main stream after it. Inside a capture the pair becomes a fork and a
+    // join of the graph. In an all-TRA frame the SMS launches, which find no
+    // work, then cost the frame nothing.
+    //
+    // Small scenes' TRA side is on the main stream, as the event between the
+    // streams would delay it. Where it fills the GPU (tra_fills) the SMS
+    // side is, so that the same delay puts its kernels first; behind the TRA
+    // blocks they run after them all (3.94M particles with 8 SMS tasks, whose
+    // kernels take 18 and 28 us: density 503 -> 497, force 485 -> 466 us launched
+    // kernel by kernel).
     cudaStream_t aux = nullptr;
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
     void fork() {
@@ -155,6 +162,13 @@ struct System {
     void join() {
         cudaEventRecord(join_ev, aux);
         cudaStreamWaitEvent(stream, join_ev, 0);
+    }
+
+    struct Sides {
+        cudaStream_t tra, sms;
+    };
+    Sides sides() const {
+        return tra_fills(fr, num_sms) ? Sides{aux, stream} : Sides{stream, aux};
     }
 
     ~System() { release(); }
@@ -186,7 +200,7 @@ struct System {
             cudaStreamDestroy(upload);
             upload = nullptr;
         }
-        for (cudaEvent_t *e : {&frames_done, &pos_up, &motion_up})
+        for (cudaEvent_t *e : {&frames_done, &pos_up, &motion_up, &sms_done})
             if (*e) {
                 cudaEventDestroy(*e);
                 *e = nullptr;
@@ -572,15 +586,19 @@ struct System {
     // pair_tasks: the arrange left the task pairing to this stage.
     void enqueue_density(int b, bool pair_tasks = false) {
         const Frame f = frame_physics(b);
+        const Sides on = sides();
         fork();
-        if (pair_tasks) launch_judge(f, max_occ, num_sms, aux);
-        launch_density(f, dp, num_sms, shape, stream, aux);
+        launch_density(f, dp, num_sms, shape, on.tra, on.sms);
+        // (the SMS passes do not read what the pairing writes)
+        if (pair_tasks) launch_judge(f, max_occ, num_sms, on.sms);
         join();
         lists_valid = true;
     }
     void enqueue_force(int b) {
+        const Frame f = frame_physics(b);
+        const Sides on = sides();
         fork();
-        launch_force(frame_physics(b), dp, num_sms, lists_valid, shape, stream, aux);
+        launch_force(f, dp, num_sms, lists_valid, shape, on.tra, on.sms);
         join();
     }
     // Force on buffer b with the integration fused in: the new state goes to
@@ -598,11 +616,12 @@ struct System {
     }
     void enqueue_force_advance(int b, bool keep_acc = true) {
         const Frame f = frame_force_advance(b, keep_acc);
+        const Sides on = sides();
         fork();
-        launch_force(f, dp, num_sms, lists_valid, shape, stream, aux);
-        // the SMS particles' keys ahead, after their force pass on the
-        // second stream (beside the TRA force pass, which hashes its own)
-        launch_hash_sms(f, f.pos_next, dp, aux);
+        launch_force(f, dp, num_sms, lists_valid, shape, on.tra, on.sms);
+        // the SMS particles' keys ahead, after their force pass (beside the
+        // TRA force pass, which hashes its own)
+        launch_hash_sms(f, f.pos_next, dp, on.sms);
         join();
         lists_valid = false;
         hashed = true;
@@ -713,24 +732,25 @@ struct System {
     gsph_status force_downloading(int b, bool keep_acc, void *const host[3]) {
         const Frame f = frame_force_advance(b, keep_acc);
         const bool split = force_in_parts(f, num_sms);
+        const Sides on = sides();
         const int units = (n + 31) / 32;
         const int ends[4] = {0, units / 8, units / 8 * 3, units};
         const float4 *src[3] = {f.pos_next, f.vel_next, f.ev_next};
         fork();
         if (split) {
-            launch_force_sms(f, dp, num_sms, shape, aux);
+            launch_force_sms(f, dp, num_sms, shape, on.sms);
         } else {
-            launch_force(f, dp, num_sms, lists_valid, shape, stream, aux);
+            launch_force(f, dp, num_sms, lists_valid, shape, on.tra, on.sms);
         }
-        launch_hash_sms(f, f.pos_next, dp, aux);
-        GSPH_CUDA(cudaEventRecord(join_ev, aux));
-        GSPH_CUDA(cudaStreamWaitEvent(xfer, join_ev, 0));   // the SMS rows, anywhere
+        launch_hash_sms(f, f.pos_next, dp, on.sms);
+        GSPH_CUDA(cudaEventRecord(sms_done, on.sms));
+        GSPH_CUDA(cudaStreamWaitEvent(xfer, sms_done, 0));   // the SMS rows, anywhere
         for (int q = split ? 0 : 2; q < 3; ++q) {
             const int first = split ? ends[q] : 0, last = ends[q + 1];
             if (split)
                 launch_force_tra_part(f, dp, num_sms, lists_valid, shape,
-                                      ForcePart{first, last, q}, stream);
-            GSPH_CUDA(cudaEventRecord(frames_done, stream));
+                                      ForcePart{first, last, q}, on.tra);
+            GSPH_CUDA(cudaEventRecord(frames_done, on.tra));
             GSPH_CUDA(cudaStreamWaitEvent(xfer, frames_done, 0));
             const size_t row = size_t(first) * 32;
             const size_t rows = std::min(size_t(last) * 32, size_t(n)) - row;
@@ -740,7 +760,7 @@ struct System {
                 if (q == 2) GSPH_CUDA(cudaEventRecord(xfer_done[k], xfer));
             }
         }
-        GSPH_CUDA(cudaStreamWaitEvent(stream, join_ev, 0));
+        join();
         lists_valid = false;
         hashed = true;
         counts_dirty = true;
@@ -1683,7 +1703,7 @@ gsph_status gsph_step_host_async(gsph_handle h, int frames, void *pos4, void *ve
         GSPH_CUDA(cudaStreamCreateWithFlags(&s.upload, cudaStreamNonBlocking));
         for (auto &e : s.xfer_done)
             GSPH_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        for (cudaEvent_t *e : {&s.frames_done, &s.pos_up, &s.motion_up})
+        for (cudaEvent_t *e : {&s.frames_done, &s.pos_up, &s.motion_up, &s.sms_done})
             GSPH_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     }
     const gsph_field fields[3] = {GSPH_FIELD_POSITION, GSPH_FIELD_VELOCITY,
