@@ -264,20 +264,33 @@ __device__ __forceinline__ void emit_cell(const Frame &f, int cell, int b, int n
 // The same for the small cells among 32 occupied cells from k0 on, by a warp:
 // eight lanes write a cell's indices side by side (one thread per cell wrote
 // to 32 sectors at a time: arrange of 3.94M particles with 8 SMS tasks 143.6 ->
-// 140.9 us), a lane its cell's tasks.
+// 140.9 us), a lane its cell's tasks. Tiles of the model without SMS cells, most
+// of them where a sparse scene has grown a few, need no cell's values (133 us).
 __device__ __forceinline__ void emit_small_cells(const Frame &f, int k0, int num_occ) {
     const int lane = threadIdx.x & 31;
     const int k = k0 + lane;
+    const int tile = k0 / kValTile;
+    const int before = f.scan_tiles4[tile].y;
+    const int after = (tile + 1) * kValTile < num_occ ? f.scan_tiles4[tile + 1].y
+                                                      : f.ctr->n_sms;
     int cell = 0, b = 0, n = 0;
-    int4 v = make_int4(0, 0, 0, 0), pre = v;
     if (k < num_occ) {
         cell = f.occ_list[k];
         b = f.cell_start[cell];
         n = f.cell_start[cell + 1] - b;
-        if (n <= kSmallCellMax) {
-            v = f.cell_val[k];
-            pre = cells_before(f, k);
-        }
+    }
+    if (before == after) {
+        // no SMS cell in the tile: its particles follow one another in the
+        // compact index, moved down by the SMS ones before them
+        const int end = __shfl_sync(0xFFFFFFFFu, b + n, min(31, num_occ - 1 - k0));
+        for (int i = __shfl_sync(0xFFFFFFFFu, b, 0) + lane; i < end; i += 32)
+            f.compact[i - before] = i;
+        return;
+    }
+    int4 v = make_int4(0, 0, 0, 0), pre = v;
+    if (k < num_occ && n <= kSmallCellMax) {
+        v = f.cell_val[k];
+        pre = cells_before(f, k);
     }
     const int middle = f.ctr->middle;
 #pragma unroll
