@@ -399,10 +399,27 @@ constexpr size_t kRowPrefetchCellBytes = size_t(64) << 20;
 // 40.4 / 38.7 at 21,952 (4.5), 43.7 / 44.8 at 32,768. Alone, the density pass
 // takes 7.9 instead of 21.2 us at 4,096 particles and the force pass 7.2
 // instead of 14.6.
-constexpr int kRowsMax1 = 5;
-constexpr int kRowsMax3 = 17;
+//
+// Between those ends the blocks per SM decide, all of which run at once. Three
+// rows per warp: from 9 units per SM (three blocks of 3 units) on, some SMs have a
+// fourth block, and a row per warp is the better one up to 11 units; from 18 on a
+// seventh. Force: an SM runs 22 warps of the small build at once and 32 of the
+// general one. The general one is better from where the small one needs a second
+// wave until it needs one itself; from 34 to 40 units both do, and the small one's
+// is the fuller. Frames, us:
+//   units per SM            8.8   9.6  10.4  12.2  17.5  18.7
+//   density, row per warp  47.3  46.8  51.5  53.6
+//   density, three rows    44.2  50.3  51.8  54.1  57.7  68.9
+//   density, general       56.7  56.1  57.4  57.9  63.6  65.7
+//   units per SM           20.0  21.3  22.7  24.2  25.7  27.3  32.4  36.1  38.1  42.2
+//   force, small           66.9  75.5  78.3  81.5  80.4  81.0  84.7  87.4  92.2 101.1
+//   force, general         73.5  75.1  76.3  78.3  76.7  81.1  80.9  90.6  95.3  98.1
+constexpr int kRowsMax1 = 5, kRowsAgain1 = 9, kRowsAgainMax1 = 11;
+constexpr int kRowsMax3 = 18;
 constexpr int kForceQuadMax = 5;
-constexpr int kForceSmallMax = 27;
+constexpr int kForceSmallMax = 21, kForceSmallAgain = 34, kForceSmallAgainMax = 40;
+// From how many units per SM a host step's force pass goes in parts.
+constexpr int kForcePartsMin = 27;
 // From how many units per SM the SMS side is put first in line (tra_fills).
 // Frame times in graphs with the TRA side first / the SMS side first, us, no SMS
 // work: 110,592 particles (23) 78.5 / 83.7, 262,144 (54) 108.0 / 109.2, 373,248
@@ -1547,7 +1564,8 @@ void launch_density_w(const Frame &f, const DevParams &P, int num_sms,
                       bool row_prefetch) {
     k_density_sms<W><<<sms_blocks(f, num_sms, shape.density_sms, W), W * 32, 0, s_sms>>>(f, P);
     const int units = (f.n + 31) / 32;
-    if (units <= num_sms * kRowsMax1)
+    if (units <= num_sms * kRowsMax1 ||
+        (units > num_sms * kRowsAgain1 && units <= num_sms * kRowsAgainMax1))
         launch_after(k_density_tra_rows<1>, units, 288, s, f, P);
     else if (units <= num_sms * kRowsMax3)
         launch_after(k_density_tra_rows<3>, (units + 2) / 3, 288, s, f, P);
@@ -1581,7 +1599,8 @@ void launch_force_tra_w(const Frame &f, const DevParams &P, int num_sms, bool fr
             <<<num_sms * shape.force_tra, W * 32, 0, s>>>(f, P, fresh, *part);
     else if (units <= num_sms * kForceQuadMax)
         k_force_tra_quad<kArt><<<units, 128, 0, s>>>(f, P, fresh);
-    else if (units <= num_sms * kForceSmallMax)
+    else if (units <= num_sms * kForceSmallMax ||
+             (units > num_sms * kForceSmallAgain && units <= num_sms * kForceSmallAgainMax))
         k_force_tra<kArt, 2, true><<<(units + 1) / 2, 64, 0, s>>>(f, P, fresh, ForcePart{});
     else
         k_force_tra<kArt, W>
@@ -1626,7 +1645,7 @@ bool tra_fills(const Frame &f, int num_sms) {
     return (f.n + 31) / 32 > num_sms * kTraFills;
 }
 bool force_in_parts(const Frame &f, int num_sms) {
-    return (f.n + 31) / 32 > num_sms * kForceSmallMax;
+    return (f.n + 31) / 32 > num_sms * kForcePartsMin;
 }
 
 void launch_force_sms(const Frame &f, const DevParams &P, int num_sms,

@@ -32,6 +32,10 @@ def state(gsph, sysm, all_tra):
 CASES = {   # particles, positions pulled together by
     "one": (1, 1.0), "quad+1": (9, 1.0), "unit-1": (31, 1.0), "unit+1": (33, 1.0), "odd": (1501, 1.0),
     "row-per-warp": (24320, 1.0), "three-rows": (24321, 1.0), "force-line": (82689, 1.0),
+    "row-per-warp again": (43777, 1.0), "three-rows again": (53505, 1.0),
+    "three-rows end": (87552, 1.0), "general density": (87553, 1.0),
+    "force-small end": (102144, 1.0), "force general": (102145, 1.0),
+    "force-small again": (165377, 1.0), "force-small again end": (194560, 1.0),
     "crowded": (2000, 0.6), "very crowded": (2000, 0.2), "crowded, three rows": (30000, 0.3),
 }
 
