@@ -356,27 +356,27 @@ __device__ __forceinline__ void move_particle(const Frame &f, int dst,
     }
 }
 
-// Velocity and evaluated velocity after a sort that moved the positions alone;
-// the pressures (ev.w) of a density pass in between stay. Two particles per
-// thread, as k_sort_small.
+// Velocity and evaluated velocity after a sort that moved the positions alone,
+// beside the density pass: the pressures that it writes (ev.w) are left out. Two
+// particles per thread, as k_sort_small.
 __global__ void __launch_bounds__(256) k_gather_motion(Frame f) {
     const int d0 = blockIdx.x * (2 * blockDim.x) + threadIdx.x;
     const int d[2] = {d0, d0 + int(blockDim.x)};
     float4 vel[2], ev[2];
-    float w[2];
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
         if (d[k] >= f.n) continue;
         const int src = f.perm[d[k]];
         vel[k] = f.vel_in[src];
         ev[k] = f.ev_in[src];
-        w[k] = f.ev[d[k]].w;
     }
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
         if (d[k] >= f.n) continue;
         f.vel[d[k]] = vel[k];
-        f.ev[d[k]] = make_float4(ev[k].x, ev[k].y, ev[k].z, w[k]);
+        float *to = reinterpret_cast<float *>(f.ev + d[k]);
+        *reinterpret_cast<float2 *>(to) = make_float2(ev[k].x, ev[k].y);
+        to[2] = ev[k].z;
     }
 }
 

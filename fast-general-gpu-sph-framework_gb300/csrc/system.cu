@@ -131,7 +131,7 @@ struct System {
     // The upload of the velocities runs on a third stream, behind that of the
     // positions, and is waited for only where the first frame needs them.
     cudaStream_t upload = nullptr;
-    cudaEvent_t pos_up = nullptr, motion_up = nullptr, sms_done = nullptr;
+    cudaEvent_t pos_up = nullptr, motion_up = nullptr, sorted = nullptr, sms_done = nullptr;
 
     void join_xfer() {
         if (!xfer_pending) return;
@@ -200,7 +200,7 @@ struct System {
             cudaStreamDestroy(upload);
             upload = nullptr;
         }
-        for (cudaEvent_t *e : {&frames_done, &pos_up, &motion_up, &sms_done})
+        for (cudaEvent_t *e : {&frames_done, &pos_up, &motion_up, &sorted, &sms_done})
             if (*e) {
                 cudaEventDestroy(*e);
                 *e = nullptr;
@@ -769,18 +769,23 @@ struct System {
     }
 
     // A frame of gsph_step_host_async, as tick(). first: the velocities are
-    // still on their way (motion_up: the upload's end) while the positions are
-    // sorted and the density pass, which needs only them, runs (1.05M particles:
-    // 917 -> 764 us a call; the gather that this adds reads and writes each
-    // velocity once). last: the state goes back to `host`.
+    // still on their way while the positions are sorted and the density pass,
+    // which needs only them, runs; they are gathered into the sorted order on
+    // the upload's stream, beside the density pass's end (1.05M particles: 917 ->
+    // 764 us a call; the gather on the main stream, after the density pass, was
+    // 8 us slower).
+    // last: the state goes back to `host`.
     gsph_status tick_host(bool first, bool last, void *const host[3]) {
         const int in = cur, out = 1 - cur;
         enqueue_arrange(in, false, !first);
-        enqueue_density(out, true);
         if (first) {
-            GSPH_CUDA(cudaStreamWaitEvent(stream, motion_up, 0));
-            launch_gather_motion(frame_arrange(in), stream);
+            GSPH_CUDA(cudaEventRecord(sorted, stream));
+            GSPH_CUDA(cudaStreamWaitEvent(upload, sorted, 0));
+            launch_gather_motion(frame_arrange(in), upload);
+            GSPH_CUDA(cudaEventRecord(motion_up, upload));
         }
+        enqueue_density(out, true);
+        if (first) GSPH_CUDA(cudaStreamWaitEvent(stream, motion_up, 0));
         gsph_status st = GSPH_OK;
         if (last)
             st = force_downloading(out, true, host);
@@ -1703,7 +1708,7 @@ gsph_status gsph_step_host_async(gsph_handle h, int frames, void *pos4, void *ve
         GSPH_CUDA(cudaStreamCreateWithFlags(&s.upload, cudaStreamNonBlocking));
         for (auto &e : s.xfer_done)
             GSPH_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        for (cudaEvent_t *e : {&s.frames_done, &s.pos_up, &s.motion_up, &s.sms_done})
+        for (cudaEvent_t *e : {&s.frames_done, &s.pos_up, &s.motion_up, &s.sorted, &s.sms_done})
             GSPH_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     }
     const gsph_field fields[3] = {GSPH_FIELD_POSITION, GSPH_FIELD_VELOCITY,
