@@ -86,8 +86,7 @@ __device__ __forceinline__ unsigned long long pack_cell(int cnt) {
     return (cnt > 0 ? (1ull << 32) : 0ull) | (unsigned long long)(unsigned)cnt;
 }
 
-__device__ __forceinline__ void load_tile_counts(const int32_t *__restrict__ in,
-                                                 int n, int first,
+__device__ __forceinline__ void load_tile_counts(const int32_t *in, int n, int first,
                                                  int (&v)[kScanItems]) {
     if (first + kScanItems <= n) {
         const int4 *p4 = reinterpret_cast<const int4 *>(in + first);
@@ -108,8 +107,7 @@ __device__ __forceinline__ void load_tile_counts(const int32_t *__restrict__ in,
 
 // Sum of every tile of kScanTile cells.
 __global__ void __launch_bounds__(kScanThreads)
-k_tile_sums(const int32_t *__restrict__ count, int numc,
-            unsigned long long *__restrict__ tiles) {
+k_tile_sums(const int32_t *count, int numc, unsigned long long *tiles) {
     chain_next();
     int v[kScanItems];
     load_tile_counts(count, numc, blockIdx.x * kScanTile + threadIdx.x * kScanItems, v);
@@ -130,7 +128,7 @@ k_tile_sums(const int32_t *__restrict__ count, int numc,
 
 // Exclusive scan of the tile sums, in place, by one block of 1,024 threads.
 __global__ void __launch_bounds__(1024)
-k_scan_tiles(unsigned long long *__restrict__ tiles, int ntiles) {
+k_scan_tiles(unsigned long long *tiles, int ntiles) {
     chain_wait();
     chain_next();
     __shared__ unsigned long long ws[32];
@@ -173,10 +171,9 @@ k_scan_tiles(unsigned long long *__restrict__ tiles, int ntiles) {
 enum class Before { kCounts, kSums, kScanned };
 template <Before kBefore>
 __global__ void __launch_bounds__(kScanThreads)
-k_cell_scan(const int32_t *__restrict__ count, int numc,
-            const unsigned long long *__restrict__ tiles,
-            int32_t *__restrict__ cell_start, int32_t *__restrict__ occ_list,
-            int32_t *__restrict__ big_list, Counters *ctr, int n_particles, int crowd) {
+k_cell_scan(const int32_t *count, int numc, const unsigned long long *tiles,
+            int32_t *cell_start, int32_t *occ_list, int32_t *big_list, Counters *ctr,
+            int n_particles, int crowd) {
     chain_wait();
     chain_next();
     const int first = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
@@ -295,10 +292,10 @@ k_scatter(Frame f, DevParams P, int model_blocks) {
     }
     const int block = blockIdx.x - model_blocks;
     const int n = f.n;
-    const uint32_t *__restrict__ key_in = f.key_in;
-    const uint32_t *__restrict__ slot = f.slot;
-    const int32_t *__restrict__ cell_start = f.cell_start;
-    unsigned long long *__restrict__ pairs = f.pairs;
+    const uint32_t *key_in = f.key_in;
+    const uint32_t *slot = f.slot;
+    const int32_t *cell_start = f.cell_start;
+    unsigned long long *pairs = f.pairs;
     if (block == 0 && threadIdx.x == 0) {
         f.ctr->num_big = f.ctr->big_fill;
         f.ctr->big_fill = 0;

@@ -210,6 +210,11 @@ inline __host__ __device__ void set_task_offset(gsph_block_task &t, int off) {
 // the kernel after it be scheduled. Both do nothing in ordinary launches. It
 // takes the launch latency out of the short kernels that follow one another
 // in a frame.
+// What the kernel before it writes is written during such a kernel's lifetime,
+// so it may not be read through a const __restrict__ pointer: that promises
+// data constant for the lifetime, and the compiler may then load it through the
+// read-only path, which chain_wait does not order. These kernels, and the
+// functions they call, take plain pointers.
 __device__ __forceinline__ void chain_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }

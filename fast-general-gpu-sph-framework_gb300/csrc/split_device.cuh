@@ -27,14 +27,14 @@ namespace gsph {
 
 namespace {
 
-__device__ __forceinline__ int cell_n(const int32_t *__restrict__ start, int c) {
+__device__ __forceinline__ int cell_n(const int32_t *start, int c) {
     return start[c + 1] - start[c];
 }
 
 // A6: SMS task count of one cell (gpu_model.cu:137-181, same neighbour
 // bounds tests; the thresholds are the reference's unless tuned), with the
 // cell's SMS and TRA particle counts: {req, sms, tra, 0}.
-__device__ __forceinline__ int4 cell_model(int gidx, const int32_t *__restrict__ start,
+__device__ __forceinline__ int4 cell_model(int gidx, const int32_t *start,
                                            const SceneTable &T, int3 thr) {
     const SceneGeom G = geom_of_cell(T, gidx);
     const int idx = gidx - G.cbase;           // the scene's own cell index
