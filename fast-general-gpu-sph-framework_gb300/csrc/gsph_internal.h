@@ -11,6 +11,7 @@
 #ifndef GSPH_INTERNAL_H_
 #define GSPH_INTERNAL_H_
 
+#include <cstddef>
 #include <cstdint>
 #include <vector>
 #include <cuda_runtime.h>
@@ -129,12 +130,12 @@ struct Counters {
     int32_t task_count;     // SMS tasks (T)
     int32_t middle;         // TRA particles
     int32_t n_sms;          // SMS particles
-    int32_t work_density;   // work counters of the persistent kernels:
-    int32_t work_force;     //   TRA units of density / force,
+    // work counters of the persistent kernels, TRA units and SMS clusters of a
+    // pass side by side (System::refill clears a pass's two words together)
+    int32_t work_density, work_density_sms;
+    int32_t work_force, work_force_sms;
     uint32_t err;           // error bits
     int32_t err_index;      // first offending particle (best effort)
-    int32_t work_density_sms;   //   SMS tasks of density / force
-    int32_t work_force_sms;
     // Set when some cell takes the SMS path this frame; when clear, every
     // particle is TRA, the compact index is the identity and the TRA/SMS
     // compaction is skipped.
@@ -146,6 +147,10 @@ struct Counters {
     int32_t work_force_part[4];   // work counters of a force pass in parts
     int32_t pad[14];
 };
+static_assert(offsetof(Counters, work_density_sms) == offsetof(Counters, work_density) + 4 &&
+                  offsetof(Counters, work_force_sms) == offsetof(Counters, work_force) + 4 &&
+                  offsetof(Counters, err_index) == offsetof(Counters, err) + 4,
+              "words that the host clears as one");
 
 // Per-frame device pointers of one batch of scenes.
 struct Frame {

@@ -107,6 +107,9 @@ struct System {
     // hold counts that no arrange will consume (cleared before a new hash).
     bool hashed = false;
     bool counts_dirty = false;
+    // The passes take their units from queues that the cell scan resets. Set
+    // by a stage call: the next one on the same grid resets its own (refill).
+    bool density_spent = false, force_spent = false;
     uint64_t frames = 0;
 
     LaunchShape shape = kMaxShape;   // CTAs per SM of the density/force kernels
@@ -582,6 +585,17 @@ struct System {
         if (pair_tasks) launch_judge(f, max_occ, num_sms, stream);
         hashed = false;          // consumed; the sort cleared the counts
         counts_dirty = false;
+        density_spent = force_spent = false;
+    }
+    // Before a stage call's pass: its queues (TRA and SMS, side by side) anew if
+    // an earlier call has used them up since the arrange, or if the launch is
+    // captured and may be replayed without one.
+    void refill(int32_t Counters::*queue, bool &spent) {
+        cudaStreamCaptureStatus captured = cudaStreamCaptureStatusNone;
+        if (!spent) cudaStreamIsCapturing(stream, &captured);
+        if (spent || captured != cudaStreamCaptureStatusNone)
+            cudaMemsetAsync(&(fr.ctr->*queue), 0, 2 * sizeof(int32_t), stream);
+        spent = true;
     }
     // pair_tasks: the arrange left the task pairing to this stage.
     void enqueue_density(int b, bool pair_tasks = false) {
@@ -1353,6 +1367,7 @@ static gsph_status need_arranged(System &s) {
 gsph_status gsph_density(gsph_handle h) {
     gsph_status st = check_handle(h);
     if (st || (st = need_arranged(h->sys))) return st;
+    h->sys.refill(&Counters::work_density, h->sys.density_spent);
     h->sys.enqueue_density(h->sys.cur);
     return h->sys.check_launch();
 }
@@ -1360,6 +1375,7 @@ gsph_status gsph_density(gsph_handle h) {
 gsph_status gsph_force(gsph_handle h) {
     gsph_status st = check_handle(h);
     if (st || (st = need_arranged(h->sys))) return st;
+    h->sys.refill(&Counters::work_force, h->sys.force_spent);
     h->sys.enqueue_force(h->sys.cur);
     return h->sys.check_launch();
 }
