@@ -961,6 +961,20 @@ __device__ __forceinline__ void force_scan(const Frame &f, const DevParams &P,
     }
 }
 
+// Start of row r's candidate range (tra_row_range's and row_range's begin), from
+// the particle's own cell `own`; a row without neighbours reads the own cell.
+__device__ __forceinline__ int row_begin(const Frame &f, const SceneGeom &G,
+                                         const MicroPos &mp, int own, int r, uint32_t mask) {
+    const int left = mp.cx > 0 ? 1 : 0;
+    const int m = mask ? own + G.gx * ((r % 3) - 1 + G.gy * ((r / 3) - 1)) : own;
+    const int s0 = f.cell_start[m - left];
+    const int s1 = f.cell_start[m];
+    const uint32_t xs = f.cell_xslab[m - left];
+    if (left && mp.lmx > 0 && xs != kXslabUnknown)
+        return s0 + min(int((xs >> (10 * (mp.lmx - 1))) & 1023u), s1 - s0);
+    return s0;
+}
+
 // The neighbours the density pass found, in the same order (rows in sequence,
 // set bits in increasing candidate index). Each lane stages its 9 (row start,
 // mask) pairs in shared memory and walks all its neighbours in one loop, so
@@ -1008,16 +1022,9 @@ k_force_tra(Frame f, DevParams P, bool fresh, ForcePart part) {
 #pragma unroll
             for (int r = 0; r < 9; ++r) mk[r] = masks[r * 32];
             const int own = G.cbase + mp.cx + G.gx * (mp.cy + G.gy * mp.cz);
-            const int left = mp.cx > 0 ? 1 : 0;
 #pragma unroll
             for (int r = 0; r < 9; ++r) {
-                const int m = mk[r] ? own + G.gx * ((r % 3) - 1 + G.gy * ((r / 3) - 1)) : own;
-                const int s0 = f.cell_start[m - left];
-                const int s1 = f.cell_start[m];
-                const uint32_t xs = f.cell_xslab[m - left];
-                int start = s0;
-                if (left && mp.lmx > 0 && xs != kXslabUnknown)
-                    start = s0 + min(int((xs >> (10 * (mp.lmx - 1))) & 1023u), s1 - s0);
+                const int start = row_begin(f, G, mp, own, r, mk[r]);
                 row_mask[r][threadIdx.x] = mk[r];
                 row_start[r][threadIdx.x] = start;
             }
@@ -1094,7 +1101,7 @@ k_force_tra(Frame f, DevParams P, bool fresh, ForcePart part) {
 // hands through shared memory so that each lane keeps one of the four sums
 // (pressure, viscosity, gradient, laplacian) and adds its terms in neighbour
 // order with k_force_tra's operations: the same bits.
-constexpr int kQuadList = 64;   // neighbours listed; with more the first lane scans
+constexpr int kQuadList = 64;   // neighbours listed; with more the first lane walks all
 template <bool kArt>
 __global__ void __launch_bounds__(128)
 k_force_tra_quad(Frame f, DevParams P, bool fresh) {
@@ -1120,19 +1127,12 @@ k_force_tra_quad(Frame f, DevParams P, bool fresh) {
     uint32_t mk[3];
     int start[3], cnt[3];
     const int own = G.cbase + mp.cx + G.gx * (mp.cy + G.gy * mp.cz);
-    const int left = mp.cx > 0 ? 1 : 0;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const int r = s + 4 * k;
         mk[k] = listed && r < 9 ? masks[r * 32] : 0u;
         cnt[k] = __popc(mk[k]);
-        const int m = mk[k] ? own + G.gx * ((r % 3) - 1 + G.gy * ((r / 3) - 1)) : own;
-        const int s0 = f.cell_start[m - left];
-        const int s1 = f.cell_start[m];
-        const uint32_t xs = f.cell_xslab[m - left];
-        start[k] = s0;
-        if (left && mp.lmx > 0 && xs != kXslabUnknown)
-            start[k] = s0 + min(int((xs >> (10 * (mp.lmx - 1))) & 1023u), s1 - s0);
+        start[k] = row_begin(f, G, mp, own, r, mk[k]);
     }
     int ahead = 0;
 #pragma unroll
@@ -1194,7 +1194,20 @@ k_force_tra_quad(Frame f, DevParams P, bool fresh) {
     a.gz = __shfl_down_sync(kFull, az, 2);
     a.lap = __shfl_down_sync(kFull, ax, 3);
     if (s != 0 || !active) return;
-    if (!listed) force_scan<kArt>(f, P, G, mp, p, pev, a);   // (the sums are zero)
+    if (!listed) {   // (the sums are zero)
+        if (found < 0) {
+            force_scan<kArt>(f, P, G, mp, p, pev, a);
+        } else {   // the masks decide, as in k_force_tra: the scan's test rounds otherwise
+            for (int r = 0; r < 9; ++r) {
+                const uint32_t mask = masks[r * 32];
+                const int from = row_begin(f, G, mp, own, r, mask);
+                for (uint32_t m = mask; m; m &= m - 1u) {
+                    const int at_j = from + __ffs(m) - 1;
+                    force_pair<false, kArt>(p, pev, f.pos[at_j], f.ev[at_j], P, a);
+                }
+            }
+        }
+    }
     write_force(f, P, self, p, pev, G, a, false);
 }
 
