@@ -1158,22 +1158,21 @@ k_force_tra_quad(Frame f, DevParams P, bool fresh) {
     int j = s < n ? list[warp][pl][s] : self;
     float4 q = f.pos[j], e = f.ev[j];
     for (int k = 0; k < rounds; ++k) {
-        const bool valid = 4 * k + s < n;
         const float4 cq = q, ce = e;
         const int next = 4 * (k + 1) + s;
         j = next < n ? list[warp][pl][next] : self;
         q = f.pos[j];
         e = f.ev[j];
         const PairTerms t = pair_terms<kArt>(p, pev, cq, ce, P);
-        *reinterpret_cast<float4 *>(mine) =
-            make_float4(t.rx, t.ry, t.rz, valid ? -t.ps : 0.f);
-        *reinterpret_cast<float4 *>(mine + 4) =
-            make_float4(t.ux, t.uy, t.uz, valid ? t.wk : 0.f);
-        *reinterpret_cast<float4 *>(mine + 8) =
-            make_float4(t.lf, valid ? t.gw : 0.f, valid ? t.wh : 0.f, 0.f);
+        *reinterpret_cast<float4 *>(mine) = make_float4(t.rx, t.ry, t.rz, -t.ps);
+        *reinterpret_cast<float4 *>(mine + 4) = make_float4(t.ux, t.uy, t.uz, t.wk);
+        *reinterpret_cast<float4 *>(mine + 8) = make_float4(t.lf, t.gw, t.wh, 0.f);
         __syncwarp();
+        // terms past the particle's neighbours (of a lane paired with itself) are
+        // skipped, not weighted by zero: the velocity may not be finite
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
+            if (4 * k + i >= n) continue;
             const float4 v = *reinterpret_cast<const float4 *>(vec + 12 * i);
             const float w = fac[12 * i];
             ax = __fmaf_rn(v.x, w, ax);
