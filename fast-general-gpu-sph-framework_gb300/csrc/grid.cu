@@ -258,6 +258,7 @@ k_cell_scan(const int32_t *count, int numc, const unsigned long long *tiles,
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == kScanThreads - 1) {
         cell_start[numc] = int32_t(run & 0xFFFFFFFFull);
         ctr->num_occ = int32_t(run >> 32);
+        ctr->num_big = 0;   // (the scatter, not launched without particles, counts them)
         ctr->work_density = 0;
         ctr->work_force = 0;
         ctr->work_density_sms = 0;
