@@ -340,6 +340,9 @@ struct LaunchShape {
     int warps;   // warps per block: 8, or 4 (then up to twice the CTAs per SM)
 };
 constexpr LaunchShape kMaxShape = {6, 4, 4, 4, 8};   // the kernels' launch bounds
+// What the launches of f's scenes take from a shape: two shapes with the same
+// answer launch the same (small scenes' TRA kernels have a shape of their own).
+LaunchShape launched_shape(const Frame &f, int num_sms, LaunchShape shape);
 
 // Shared-memory carveouts of the density and force kernels (once per
 // device, before their first launch).

@@ -1575,16 +1575,36 @@ int sms_blocks(const Frame &f, int num_sms, int ctas, int warps) {
     return num_sms * (need <= 2 ? std::min(need, ctas) : ctas);
 }
 
+// Which build the TRA passes of a scene of f.n particles run (kRowsMax1 and the
+// following lines). All but the general ones have a fixed shape.
+enum class DensityTra { kRow1, kRow3, kGeneral };
+DensityTra density_build(const Frame &f, int num_sms) {
+    const int units = (f.n + 31) / 32;
+    if (units <= num_sms * kRowsMax1 ||
+        (units > num_sms * kRowsAgain1 && units <= num_sms * kRowsAgainMax1))
+        return DensityTra::kRow1;
+    return units <= num_sms * kRowsMax3 ? DensityTra::kRow3 : DensityTra::kGeneral;
+}
+enum class ForceTra { kQuad, kSmall, kGeneral };
+ForceTra force_build(const Frame &f, int num_sms) {
+    const int units = (f.n + 31) / 32;
+    if (units <= num_sms * kForceQuadMax) return ForceTra::kQuad;
+    return units <= num_sms * kForceSmallMax ||
+                   (units > num_sms * kForceSmallAgain && units <= num_sms * kForceSmallAgainMax)
+               ? ForceTra::kSmall
+               : ForceTra::kGeneral;
+}
+
 template <int W>
 void launch_density_w(const Frame &f, const DevParams &P, int num_sms,
                       const LaunchShape &shape, cudaStream_t s, cudaStream_t s_sms,
                       bool row_prefetch) {
     k_density_sms<W><<<sms_blocks(f, num_sms, shape.density_sms, W), W * 32, 0, s_sms>>>(f, P);
     const int units = (f.n + 31) / 32;
-    if (units <= num_sms * kRowsMax1 ||
-        (units > num_sms * kRowsAgain1 && units <= num_sms * kRowsAgainMax1))
+    const DensityTra build = density_build(f, num_sms);
+    if (build == DensityTra::kRow1)
         launch_after(k_density_tra_rows<1>, units, 288, s, f, P);
-    else if (units <= num_sms * kRowsMax3)
+    else if (build == DensityTra::kRow3)
         launch_after(k_density_tra_rows<3>, (units + 2) / 3, 288, s, f, P);
     else {
         const bool many = f.scenes.count > 1;
@@ -1611,13 +1631,13 @@ template <bool kArt, int W>
 void launch_force_tra_w(const Frame &f, const DevParams &P, int num_sms, bool fresh,
                         const LaunchShape &shape, const ForcePart *part, cudaStream_t s) {
     const int units = (f.n + 31) / 32;
+    const ForceTra build = force_build(f, num_sms);
     if (part)
         k_force_tra<kArt, W, false, true>
             <<<num_sms * shape.force_tra, W * 32, 0, s>>>(f, P, fresh, *part);
-    else if (units <= num_sms * kForceQuadMax)
+    else if (build == ForceTra::kQuad)
         k_force_tra_quad<kArt><<<units, 128, 0, s>>>(f, P, fresh);
-    else if (units <= num_sms * kForceSmallMax ||
-             (units > num_sms * kForceSmallAgain && units <= num_sms * kForceSmallAgainMax))
+    else if (build == ForceTra::kSmall)
         k_force_tra<kArt, 2, true><<<(units + 1) / 2, 64, 0, s>>>(f, P, fresh, ForcePart{});
     else
         k_force_tra<kArt, W>
@@ -1656,6 +1676,14 @@ void launch_density(const Frame &f, const DevParams &P, int num_sms,
         launch_density_w<kWarpsPerBlock / 2>(f, P, num_sms, shape, s, s_sms, row_prefetch);
     else
         launch_density_w<kWarpsPerBlock>(f, P, num_sms, shape, s, s_sms, row_prefetch);
+}
+
+LaunchShape launched_shape(const Frame &f, int num_sms, LaunchShape shape) {
+    if (density_build(f, num_sms) != DensityTra::kGeneral) shape.density_tra = 0;
+    if (force_build(f, num_sms) != ForceTra::kGeneral) shape.force_tra = 0;
+    shape.density_sms = sms_blocks(f, num_sms, shape.density_sms, shape.warps);
+    shape.force_sms = sms_blocks(f, num_sms, shape.force_sms, shape.warps);
+    return shape;
 }
 
 bool tra_fills(const Frame &f, int num_sms) {

@@ -917,9 +917,27 @@ struct System {
         return GSPH_OK;
     }
 
+    // Whether two tunings make the same launches for the current scenes.
+    bool same_launches(const gsph_tuning &a, const gsph_tuning &b) const {
+        if (a.sparse_total != b.sparse_total || a.sparse_self != b.sparse_self ||
+            a.mid_total != b.mid_total)
+            return false;
+        auto of = [&](const gsph_tuning &t) {
+            return launched_shape(fr, num_sms,
+                                  {t.ctas_density_tra, t.ctas_density_sms, t.ctas_force_tra,
+                                   t.ctas_force_sms,
+                                   t.warps_per_block ? t.warps_per_block : kMaxShape.warps});
+        };
+        const LaunchShape x = of(a), y = of(b);
+        return x.density_tra == y.density_tra && x.density_sms == y.density_sms &&
+               x.force_tra == y.force_tra && x.force_sms == y.force_sms && x.warps == y.warps;
+    }
+
     // Times each candidate on a saved copy of the current state (one warm-up
     // frame, then `trial` frames between events), restores the state after
-    // every trial and installs the fastest candidate.
+    // every trial and installs the fastest candidate. Of candidates that make
+    // the same launches only the first is tried: between the others only noise
+    // would choose.
     gsph_status autotune(int trial, const gsph_tuning *cand, int nc, gsph_tuning *best,
                          float *best_ms) {
         if (trial < 1 || nc < 1 || !cand) {
@@ -980,6 +998,9 @@ struct System {
             graph_frames = 0;
             timing = false;
             for (int k = 0; k < nc && !st; ++k) {
+                bool tried = false;
+                for (int j = 0; j < k && !tried; ++j) tried = same_launches(cand[j], cand[k]);
+                if (tried) continue;
                 if ((st = restore()) || (st = set_tuning(cand[k])) || (st = tick())) break;
                 cudaEventRecord(e0, stream);
                 for (int f = 0; f < trial && !st; ++f) st = tick();

@@ -154,7 +154,12 @@ typedef struct {
  * most 6 / 4 / 4 / 4 with 8 warps per block, twice that with 4; the blocks of
  * 4 warps are the same kernels built for that shape). Other thresholds change which
  * cells take the SMS path: results stay within the parity tolerances but the
- * split is no longer the reference's. */
+ * split is no longer the reference's.
+ * Small scenes run TRA kernels of a fixed shape, which ignore the TRA counts
+ * and warps_per_block: density up to about 18 work units (32 particles) per SM,
+ * force up to about 21 and from 34 to 40 (on 152 SMs 87,000, 102,000 and 165,000
+ * to 194,000 particles). The SMS passes launch fewer blocks than asked for
+ * where the scene has too few particles to fill them. */
 typedef struct {
     int32_t sparse_total, sparse_self, mid_total;
     int32_t ctas_density_tra, ctas_density_sms, ctas_force_tra, ctas_force_sms;
@@ -405,7 +410,8 @@ gsph_status gsph_set_viscosity_model(gsph_handle h, int model, float alpha, floa
 /* Times n_candidates tunings (NULL: a built-in grid of split thresholds and
  * CTAs per SM) on the handle's current state, frames_per_trial frames each
  * after one warm-up frame, restoring the state after every trial, and
- * installs the fastest. best_out / best_ms_out (either may be NULL) receive
+ * installs the fastest. Candidates that would launch what an earlier one
+ * launches (see gsph_tuning) are not tried again. best_out / best_ms_out (either may be NULL) receive
  * it and its device time per frame. The state, frame counter and results of
  * the handle are as before the call. Replaces the reference's fixed
  * thresholds; no counterpart in the reference. */
