@@ -363,7 +363,7 @@ bool force_in_parts(const Frame &f, int num_sms);
 // The force pass's two sides by themselves, and a part of the TRA side: the particles
 // [32 begin, 32 end) of the compact index, so that all TRA particles among the
 // first 32 end sorted ones are done after the parts up to it. Parts (at most 4,
-// `queue` their number) suit scenes past the small-scene builds.
+// `queue` their number) suit scenes past kForcePartsMin.
 struct ForcePart {
     int begin, end, queue;
 };

@@ -418,8 +418,13 @@ constexpr int kRowsMax1 = 5, kRowsAgain1 = 9, kRowsAgainMax1 = 11;
 constexpr int kRowsMax3 = 18;
 constexpr int kForceQuadMax = 5;
 constexpr int kForceSmallMax = 21, kForceSmallAgain = 34, kForceSmallAgainMax = 40;
-// From how many units per SM a host step's force pass goes in parts.
-constexpr int kForcePartsMin = 27;
+// From how many units per SM a host step's force pass goes in parts
+// (System::force_downloading): a part costs launches and a tail, and has to be worth
+// it. Host steps, us, whole / in parts:
+//   units per SM          27       44       54       65       77       90      105      206
+//   one at a time    169/197  208/218  235/246  262/268  298/296  336/324  379/355  663/599
+//   queued           139/171  176/196  193/219  215/241  240/258  265/280  299/307  530/512
+constexpr int kForcePartsMin = 76;
 // From how many units per SM the SMS side is put first in line (tra_fills).
 // Frame times in graphs with the TRA side first / the SMS side first, us, no SMS
 // work: 110,592 particles (23) 78.5 / 83.7, 262,144 (54) 108.0 / 109.2, 373,248

@@ -741,8 +741,7 @@ struct System {
     // waits for, and every part costs a tail: 3.94M particles, calls back to
     // back, 1,776 us with these parts, 1,859 with 1/8 + 3/8 + 1/2, 1,840 with
     // 1/16 + 3/16 + 3/4, 1,965 with 1/4 + 3/8 + 3/8, 1,940 in one piece; 1.05M, one
-    // call at a time, 764 -> 684 us. Scenes of the small-scene builds go back
-    // whole.
+    // call at a time, 764 -> 684 us. Smaller scenes (kForcePartsMin) go back whole.
     gsph_status force_downloading(int b, bool keep_acc, void *const host[3]) {
         const Frame f = frame_force_advance(b, keep_acc);
         const bool split = force_in_parts(f, num_sms);
