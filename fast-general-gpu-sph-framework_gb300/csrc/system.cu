@@ -741,10 +741,24 @@ struct System {
     // waits for, and every part costs a tail: 3.94M particles, calls back to
     // back, 1,776 us with these parts, 1,859 with 1/8 + 3/8 + 1/2, 1,840 with
     // 1/16 + 3/16 + 3/4, 1,965 with 1/4 + 3/8 + 3/8, 1,940 in one piece; 1.05M, one
-    // call at a time, 764 -> 684 us. Smaller scenes (kForcePartsMin) go back whole.
-    gsph_status force_downloading(int b, bool keep_acc, void *const host[3]) {
+    // call at a time, 764 -> 684 us. Smaller scenes (kForcePartsMin) go back whole,
+    // and so do arrays that are not pinned: a copy into those keeps the host until
+    // it is done, and with it the next part's launch (1M particles 982 us in parts,
+    // 884 whole; 913 with all copies before and after the frame).
+    bool in_parts(void *const host[3]) const {
+        if (!force_in_parts(fr, num_sms)) return false;
+        for (int k = 0; k < 3; ++k) {
+            cudaPointerAttributes attr{};
+            if (cudaPointerGetAttributes(&attr, host[k]) != cudaSuccess) {
+                cudaGetLastError();
+                return false;
+            }
+            if (attr.type == cudaMemoryTypeUnregistered) return false;
+        }
+        return true;
+    }
+    gsph_status force_downloading(int b, bool keep_acc, void *const host[3], bool split) {
         const Frame f = frame_force_advance(b, keep_acc);
-        const bool split = force_in_parts(f, num_sms);
         const Sides on = sides();
         const int units = (n + 31) / 32;
         const int ends[4] = {0, units / 8, units / 8 * 3, units};
@@ -787,8 +801,8 @@ struct System {
     // the upload's stream, beside the density pass's end (1.05M particles: 917 ->
     // 764 us a call; the gather on the main stream, after the density pass, was
     // 8 us slower).
-    // last: the state goes back to `host`.
-    gsph_status tick_host(bool first, bool last, void *const host[3]) {
+    // last: the state goes back to `host`, in parts if `split`.
+    gsph_status tick_host(bool first, bool last, void *const host[3], bool split) {
         const int in = cur, out = 1 - cur;
         enqueue_arrange(in, false, !first);
         if (first) {
@@ -801,7 +815,7 @@ struct System {
         if (first) GSPH_CUDA(cudaStreamWaitEvent(stream, motion_up, 0));
         gsph_status st = GSPH_OK;
         if (last)
-            st = force_downloading(out, true, host);
+            st = force_downloading(out, true, host, split);
         else
             enqueue_force_advance(out, false);
         if (!st) st = check_launch();
@@ -1751,6 +1765,7 @@ gsph_status gsph_step_host_async(gsph_handle h, int frames, void *pos4, void *ve
                                   GSPH_FIELD_EVAL_VELOCITY};
     void *host[3] = {pos4, vel4, ev4};
     const size_t bytes = size_t(s.n) * sizeof(float4);
+    const bool split = s.in_parts(host);
     // upload: each array after its previous return copy (if any) is done; the
     // velocities behind the positions, beside the first frame's work on these
     for (int k = 0; k < 3; ++k) {
@@ -1773,9 +1788,9 @@ gsph_status gsph_step_host_async(gsph_handle h, int frames, void *pos4, void *ve
     // the last of them
     const bool graphs = s.graph_frames > 0 && frames >= s.graph_frames;
     if (frames > 0 && bytes && !graphs && !s.timing) {
-        if ((st = s.tick_host(true, frames == 1, host))) return st;
+        if ((st = s.tick_host(true, frames == 1, host, split))) return st;
         for (int k = 1; k < frames; ++k)
-            if ((st = s.tick_host(false, k == frames - 1, host))) return st;
+            if ((st = s.tick_host(false, k == frames - 1, host, split))) return st;
         return GSPH_OK;
     }
     GSPH_CUDA(cudaStreamWaitEvent(s.stream, s.motion_up, 0));

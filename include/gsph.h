@@ -370,7 +370,8 @@ gsph_status gsph_copy_out_async(gsph_handle h, gsph_field field,
  * same arrays (HybridSystem::tick with the state kept on the host). Asynchronous:
  * the arrays are complete after gsph_sync. Both ways run on internal streams:
  * the velocities go up beside the first frame's sort and density pass, the state
- * of a large scene goes back in parts while the last force pass still runs, and
+ * of a large scene goes back in parts while the last force pass still runs (not
+ * into arrays that are not pinned: they work, but keep the host), and
  * the next call's upload of an array waits only for that array's own download;
  * every other call on the handle first waits for all of them. */
 gsph_status gsph_step_host_async(gsph_handle h, int frames, void *pos4, void *vel4,
