@@ -339,9 +339,7 @@ struct LaunchShape {
     int density_tra, density_sms, force_tra, force_sms;
     int warps;   // warps per block: 8, or 4 (then up to twice the CTAs per SM)
 };
-// What a shape may ask for with 8 warps: the kernels' launch bounds, but for the SMS
-// force pass, which holds and launches 3 at most (kForceSmsCtas).
-constexpr LaunchShape kMaxShape = {6, 4, 4, 4, 8};
+constexpr LaunchShape kMaxShape = {6, 4, 4, 4, 8};   // the kernels' launch bounds
 // What the launches of f's scenes take from a shape: two shapes with the same
 // answer launch the same (small scenes' TRA kernels have a shape of their own).
 LaunchShape launched_shape(const Frame &f, int num_sms, LaunchShape shape);

@@ -697,12 +697,14 @@ __device__ __forceinline__ ClusterBox cluster_box(const float4 &p, uint32_t key)
 // 128); else they come from the queue. Negative: done.
 struct ClusterUnits {
     int count, per, own;
-    // blocks: the grid's, all of which run at once
+    // blocks: those of the grid that run at once
     __device__ __forceinline__ ClusterUnits(int units, int warps, int blocks)
         : count(units) {
         per = (units + blocks - 1) / blocks;
         const int warp = threadIdx.x >> 5;
-        own = per > warps ? -2 : warp < per ? int(blockIdx.x) * per + warp : -1;
+        own = per > warps ? -2
+              : warp < per && int(blockIdx.x) < blocks ? int(blockIdx.x) * per + warp
+                                                       : -1;
     }
     __device__ __forceinline__ int next(int *queue) {
         int u = own;
@@ -1228,7 +1230,7 @@ static_assert(kForceCluster == kDenCluster, "sms_blocks counts one cluster size"
 constexpr int kForceSmsCtas = 3;   // resident blocks per SM
 template <bool kArt, int W>
 __global__ void __launch_bounds__(W * 32, kForceSmsCtas * kWarpsPerBlock / W)
-k_force_sms(Frame f, DevParams P) {
+k_force_sms(Frame f, DevParams P, int resident) {
     constexpr int C = kForceCluster, kGroups = 32 / C;
     // candidate pair k (slots 2k, 2k+1) as four float4s: (x, x, y, y),
     // (z, z, 1/rho, 1/rho), (vx, vx, vy, vy), (vz, vz, p, p)
@@ -1240,7 +1242,7 @@ k_force_sms(Frame f, DevParams P) {
     if (task_count == 0) return;   // no SMS work: skip the queue atomics
     float4 *sa = sm[0][warp], *sb4 = sm[1][warp], *sc = sm[2][warp], *sd = sm[3][warp];
     const int i = lane % C, g = lane / C;
-    ClusterUnits units(task_count * kGroups, W, gridDim.x);
+    ClusterUnits units(task_count * kGroups, W, min(int(gridDim.x), resident));
     for (int u; (u = units.next(&f.ctr->work_force_sms)) >= 0;) {
         const gsph_block_task task = f.tasks[u / kGroups];
         const int first = task.cell_begin + task_offset(task) + (u % kGroups) * C;
@@ -1622,16 +1624,11 @@ void launch_density_w(const Frame &f, const DevParams &P, int num_sms,
     }
 }
 
-// The SMS force pass holds fewer blocks per SM than a shape may ask for.
-int force_sms_blocks(const Frame &f, int num_sms, int ctas, int warps) {
-    return sms_blocks(f, num_sms, std::min(ctas, kForceSmsCtas * kWarpsPerBlock / warps), warps);
-}
-
 template <bool kArt, int W>
 void launch_force_sms_w(const Frame &f, const DevParams &P, int num_sms,
                         const LaunchShape &shape, cudaStream_t s) {
-    k_force_sms<kArt, W><<<force_sms_blocks(f, num_sms, shape.force_sms, W), W * 32, 0, s>>>(
-        f, P);
+    k_force_sms<kArt, W><<<sms_blocks(f, num_sms, shape.force_sms, W), W * 32, 0, s>>>(
+        f, P, num_sms * kForceSmsCtas * kWarpsPerBlock / W);
 }
 
 // part: null for all units.
@@ -1690,7 +1687,7 @@ LaunchShape launched_shape(const Frame &f, int num_sms, LaunchShape shape) {
     if (density_build(f, num_sms) != DensityTra::kGeneral) shape.density_tra = 0;
     if (force_build(f, num_sms) != ForceTra::kGeneral) shape.force_tra = 0;
     shape.density_sms = sms_blocks(f, num_sms, shape.density_sms, shape.warps);
-    shape.force_sms = force_sms_blocks(f, num_sms, shape.force_sms, shape.warps);
+    shape.force_sms = sms_blocks(f, num_sms, shape.force_sms, shape.warps);
     return shape;
 }
 

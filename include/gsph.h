@@ -159,9 +159,7 @@ typedef struct {
  * and warps_per_block: density up to about 18 work units (32 particles) per SM,
  * force up to about 21 and from 34 to 40 (on 152 SMs 87,000, 102,000 and 165,000
  * to 194,000 particles). The SMS passes launch fewer blocks than asked for
- * where the scene has too few particles to fill them, and the SMS force pass
- * never more than 3 per SM with 8 warps (6 with 4), which is what an SM holds:
- * a count of 4 (8) is taken and acts as 3 (6). */
+ * where the scene has too few particles to fill them. */
 typedef struct {
     int32_t sparse_total, sparse_self, mid_total;
     int32_t ctas_density_tra, ctas_density_sms, ctas_force_tra, ctas_force_sms;
