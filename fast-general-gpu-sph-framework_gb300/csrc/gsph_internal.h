@@ -339,7 +339,9 @@ struct LaunchShape {
     int density_tra, density_sms, force_tra, force_sms;
     int warps;   // warps per block: 8, or 4 (then up to twice the CTAs per SM)
 };
-constexpr LaunchShape kMaxShape = {6, 4, 4, 4, 8};   // the kernels' launch bounds
+// The most a shape may ask for: the kernels' launch bounds, but for the SMS force
+// pass, of which an SM holds three blocks (kForceSmsCtas).
+constexpr LaunchShape kMaxShape = {6, 4, 4, 4, 8};
 // What the launches of f's scenes take from a shape: two shapes with the same
 // answer launch the same (small scenes' TRA kernels have a shape of their own).
 LaunchShape launched_shape(const Frame &f, int num_sms, LaunchShape shape);

@@ -1227,7 +1227,11 @@ k_force_tra_quad(Frame f, DevParams P, bool fresh) {
 // are added at the end.
 constexpr int kForceCluster = 16;
 static_assert(kForceCluster == kDenCluster, "sms_blocks counts one cluster size");
-constexpr int kForceSmsCtas = 3;   // resident blocks per SM
+// Resident blocks per SM. The grid may hold a fourth (kMaxShape), which starts
+// when another leaves and finds the queue empty; a grid of three is no faster in
+// dense scenes and slower where there is no SMS work (46,656 particles all TRA
+// 50.0 us a frame against 46.7, from 110,592 on the same).
+constexpr int kForceSmsCtas = 3;
 template <bool kArt, int W>
 __global__ void __launch_bounds__(W * 32, kForceSmsCtas * kWarpsPerBlock / W)
 k_force_sms(Frame f, DevParams P, int resident) {

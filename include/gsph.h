@@ -159,7 +159,9 @@ typedef struct {
  * and warps_per_block: density up to about 18 work units (32 particles) per SM,
  * force up to about 21 and from 34 to 40 (on 152 SMs 87,000, 102,000 and 165,000
  * to 194,000 particles). The SMS passes launch fewer blocks than asked for
- * where the scene has too few particles to fill them. */
+ * where the scene has too few particles to fill them, and an SM holds three
+ * blocks of 8 warps (six of 4) of the SMS force pass at a time: more may be
+ * asked for, and start when others leave. */
 typedef struct {
     int32_t sparse_total, sparse_self, mid_total;
     int32_t ctas_density_tra, ctas_density_sms, ctas_force_tra, ctas_force_sms;
