@@ -1039,9 +1039,8 @@ k_force_tra(Frame f, DevParams P, bool fresh, ForcePart part) {
             // two (kSmall: four) neighbours per iteration: their loads are in
             // flight before the first pair is evaluated (the order of the sums
             // is unchanged)
-            int k = 0;
             if constexpr (kSmall) {
-                for (; k < found; k += 4) {
+                for (int k = 0; k < found; k += 4) {
                     float4 q[4], e[4];
 #pragma unroll
                     for (int s = 0; s < 4; ++s) {
@@ -1062,35 +1061,37 @@ k_force_tra(Frame f, DevParams P, bool fresh, ForcePart part) {
                     for (int s = 0; s < 4; ++s)
                         if (k + s < found) force_pair<false, kArt>(p, pev, q[s], e[s], P, a);
                 }
-            }
-            for (; k + 1 < found; k += 2) {
-                while (!mask) {
-                    ++r;
-                    mask = row_mask[r][threadIdx.x];
-                    base = row_start[r][threadIdx.x];
+            } else {
+                int k = 0;
+                for (; k + 1 < found; k += 2) {
+                    while (!mask) {
+                        ++r;
+                        mask = row_mask[r][threadIdx.x];
+                        base = row_start[r][threadIdx.x];
+                    }
+                    const int j0 = base + __ffs(mask) - 1;
+                    mask &= mask - 1u;
+                    while (!mask) {
+                        ++r;
+                        mask = row_mask[r][threadIdx.x];
+                        base = row_start[r][threadIdx.x];
+                    }
+                    const int j1 = base + __ffs(mask) - 1;
+                    mask &= mask - 1u;
+                    const float4 q0 = f.pos[j0], e0 = f.ev[j0];
+                    const float4 q1 = f.pos[j1], e1 = f.ev[j1];
+                    force_pair<false, kArt>(p, pev, q0, e0, P, a);
+                    force_pair<false, kArt>(p, pev, q1, e1, P, a);
                 }
-                const int j0 = base + __ffs(mask) - 1;
-                mask &= mask - 1u;
-                while (!mask) {
-                    ++r;
-                    mask = row_mask[r][threadIdx.x];
-                    base = row_start[r][threadIdx.x];
+                if (k < found) {
+                    while (!mask) {
+                        ++r;
+                        mask = row_mask[r][threadIdx.x];
+                        base = row_start[r][threadIdx.x];
+                    }
+                    const int j = base + __ffs(mask) - 1;
+                    force_pair<false, kArt>(p, pev, f.pos[j], f.ev[j], P, a);
                 }
-                const int j1 = base + __ffs(mask) - 1;
-                mask &= mask - 1u;
-                const float4 q0 = f.pos[j0], e0 = f.ev[j0];
-                const float4 q1 = f.pos[j1], e1 = f.ev[j1];
-                force_pair<false, kArt>(p, pev, q0, e0, P, a);
-                force_pair<false, kArt>(p, pev, q1, e1, P, a);
-            }
-            if (k < found) {
-                while (!mask) {
-                    ++r;
-                    mask = row_mask[r][threadIdx.x];
-                    base = row_start[r][threadIdx.x];
-                }
-                const int j = base + __ffs(mask) - 1;
-                force_pair<false, kArt>(p, pev, f.pos[j], f.ev[j], P, a);
             }
         } else {
             force_scan<kArt>(f, P, G, mp, p, pev, a);
