@@ -387,36 +387,34 @@ __device__ __forceinline__ void write_force(const Frame &f, const DevParams &P,
 constexpr size_t kRowPrefetchCellBytes = size_t(64) << 20;
 
 // Up to how many work units (32 particles) per SM the small-scene builds run:
-// k_density_tra_rows with a row per warp and with three rows per warp, and
-// the small build of k_force_tra. Frame times (CUDA graphs, 152 SMs), the
-// general builds against the small ones, us:
-//   particles (units per SM)    4,096 (0.8)  32,768 (6.7)  64,000 (13)  110,592 (23)  262,144 (54)
-//   density, a row per warp       58 / 45       65 / 54      70 / 67       80 / 87      124 / 162
-//   density, three rows           58 / 47       65 / 52      70 / 65       80 / 82      124 / 147
-//   force                         58 / 56       72 / 65      79 / 71       86 / 80      119 / 123
-// (each line with the other pass fixed). Four lanes per particle in the force
-// (k_force_tra_quad) against that small build: 34.6 / 29.2 at 4,096 particles,
-// 40.4 / 38.7 at 21,952 (4.5), 43.7 / 44.8 at 32,768. Alone, the density pass
-// takes 7.9 instead of 21.2 us at 4,096 particles and the force pass 7.2
-// instead of 14.6.
-//
-// Between those ends the blocks per SM decide, all of which run at once. Three
-// rows per warp: from 9 units per SM (three blocks of 3 units) on, some SMs have a
-// fourth block, and a row per warp is the better one up to 11 units; from 18 on a
-// seventh. Force: an SM runs 22 warps of the small build at once and 32 of the
-// general one. The general one is better from where the small one needs a second
-// wave until it needs one itself; from 34 to 40 units both do, and the small one's
-// is the fuller. Frames, us:
-//   units per SM            8.8   9.6  10.4  12.2  17.5  18.7
-//   density, row per warp  47.3  46.8  51.5  53.6
-//   density, three rows    44.2  50.3  51.8  54.1  57.7  68.9
-//   density, general       56.7  56.1  57.4  57.9  63.6  65.7
-//   units per SM           20.0  21.3  22.7  24.2  25.7  27.3  32.4  36.1  38.1  42.2
-//   force, small           66.9  75.5  78.3  81.5  80.4  81.0  84.7  87.4  92.2 101.1
-//   force, general         73.5  75.1  76.3  78.3  76.7  81.1  80.9  90.6  95.3  98.1
+// k_density_tra_rows with a row per warp and with three rows per warp, the four
+// lanes per particle of k_force_tra_quad and the small build of k_force_tra.
+// The blocks per SM decide, all of which run at once. A row per warp gives way
+// where units start to wait (5 per SM), three rows where some SMs have a fourth
+// block and the others three (9 to 11, where the single rows are ahead again), and
+// for good at a seventh (18). Force: the four lanes' blocks of 32 particles run at
+// most four to an SM without waiting. An SM runs 22 warps of the small build at
+// once and 32 of the general one: the general one is better from where the
+// small one needs a second wave until it needs one itself; from 34 to 40 units
+// both do, and the small one's is the fuller. Frames in CUDA graphs on 152 SMs,
+// the dam break, us (three runs, 0.1 to 0.5 apart):
+//   units per SM            1.6   3.6   4.5   5.0   5.6   8.8   9.6  10.4  12.2  15.2  17.5  18.7
+//   density, row per warp  28.0  31.7  38.4  40.7  41.9  47.4  46.7  51.7  53.6  59.8  63.5  66.6
+//   density, three rows    31.4  34.4  40.9  38.8  38.7  44.3  50.3  51.8  54.3  56.3  58.1  69.0
+//   density, general       44.8  49.1  55.5  52.8  53.0  56.9  56.1  57.3  58.3  61.5  63.8  66.2
+//   units per SM            1.6   3.6   4.0   4.5   5.0   5.6  13.2  17.5  20.0
+//   force, four lanes      28.0  31.0  37.6  38.2  40.7  41.0  63.0  71.4  81.3
+//   force, small           33.5  34.6  35.7  37.1  38.7  38.7  54.0  58.0  66.7
+//   force, general         36.9  39.3        41.2  43.5  43.5  60.5  65.4  72.9
+//   units per SM           21.3  22.7  25.7  28.9  32.4  34.2  36.1  38.1  40.1  42.2  44.4  53.9
+//   force, small           75.8  78.5  80.5  83.8  84.7  87.6  87.5  92.9  91.7 101.4 100.8 112.9
+//   force, general         75.5  76.5  77.0  78.7  80.7  87.8  89.7  95.2  92.2  98.0  97.1 110.3
+// The same fluid in motion agrees (row per warp / three rows at 9.6 units 55.6 /
+// 59.2, at 12.2 58.2 / 57.7; four lanes / small at 4.0 37.7 / 36.6; small / general at
+// 22.7 83.0 / 80.6, at 38.1 95.4 / 99.3, at 42.2 105.7 / 103.4).
 constexpr int kRowsMax1 = 5, kRowsAgain1 = 9, kRowsAgainMax1 = 11;
 constexpr int kRowsMax3 = 18;
-constexpr int kForceQuadMax = 5;
+constexpr int kForceQuadMax = 4;
 constexpr int kForceSmallMax = 21, kForceSmallAgain = 34, kForceSmallAgainMax = 40;
 // From how many units per SM a host step's force pass goes in parts
 // (System::force_downloading): a part costs launches and a tail, and has to be worth
@@ -426,10 +424,15 @@ constexpr int kForceSmallMax = 21, kForceSmallAgain = 34, kForceSmallAgainMax = 
 //   queued           139/171  176/196  193/219  215/241  240/258  265/280  299/307  530/512
 constexpr int kForcePartsMin = 76;
 // From how many units per SM the SMS side is put first in line (tra_fills).
-// Frame times in graphs with the TRA side first / the SMS side first, us, no SMS
-// work: 110,592 particles (23) 78.5 / 83.7, 262,144 (54) 108.0 / 109.2, 373,248
-// (77) 134.8 / 135.4, 1M (206) 297.4 / 296.9, 3.94M (811) 1,047 / 1,043; 3.94M with
-// 8 SMS tasks 1,214 / 1,203.
+// Frames with the TRA side first / the SMS side first, us (three runs, 0.1 to 0.7
+// apart): in graphs, kernel by kernel, and the same for the fluid in motion, which
+// has a few SMS tasks:
+//   units per SM        54            105            140            206             811
+//   graphs        107.3/109.2    168.7/170.1    217.4/215.9    297.7/296.5   1042.8/1036.8
+//   by kernel     114.0/115.5    175.7/177.3    232.0/223.1    315.2/303.9   1071.2/1045.1
+//   motion        120.7/120.7    185.2/180.0    232.8/226.4    321.9/314.9   1124.9/1112.9
+//   by kernel     135.8/126.9    209.1/187.6    260.8/234.3    353.1/322.9   1160.9/1121.8
+// (Below the line it pays with SMS work and costs 1 to 2 us without.)
 constexpr int kTraFills = 128;
 
 // Warps per block of the density and force kernels: 8 by default; each
