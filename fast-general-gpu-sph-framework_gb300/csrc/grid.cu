@@ -11,9 +11,9 @@
 //   cell info      src/grid/sph_arrangement.cu:1342-1351 (calculate_cell_info)
 //
 // Design here (not a translation):
-//   * counting is per COARSE cell (numc ints, not numc*64), with warp-aggregated
-//     atomics (match.any) so a warp of sorted particles issues one atomic per
-//     cell it touches;
+//   * counting is per COARSE cell (numc ints, not numc*64), with one atomic for
+//     each run of a warp's lanes that lie in the same cell (in the force pass,
+//     whose particles are sorted, for each cell of the warp);
 //   * the coarse scan is reduce-then-scan (no inter-CTA waits), a single pass
 //     for small grids; it also compacts the occupied cells and the list of
 //     large cells;
@@ -37,7 +37,7 @@ namespace {
 constexpr unsigned kFull = 0xFFFFFFFFu;
 
 // ---------------------------------------------------------------------------
-// A2: key + per-coarse-cell slot (warp-aggregated atomics).
+// A2: key + per-coarse-cell slot (an atomic per run of lanes in a cell).
 __global__ void __launch_bounds__(256)
 k_hash_count(const float4 *__restrict__ pos, int n, DevParams P, SceneTable T,
              uint32_t *__restrict__ key_out, uint32_t *__restrict__ slot_out,

@@ -123,8 +123,8 @@ __device__ __forceinline__ MicroPos micro_of(float4 p, const DevParams &P,
     return r;
 }
 
-// A TRA particle's neighbour rows in three registers and the x-y strides: its
-// own cell, and in `flags` which of the nine rows lie in the grid (bits 0-8),
+// A TRA particle's neighbour rows in four registers: its own cell, the strides
+// of a cell in y and z, and in `flags` which of the nine rows lie in the grid (bits 0-8),
 // whether the left and right cells do (9, 10) and its micro-x slab (11, 12).
 // Eight registers of grid sizes and cell coordinates in the row loop cost a
 // batch 18% of the density pass (5.28M particles in 64 scenes 701 us, with this

@@ -434,7 +434,8 @@ gsph_status gsph_benchmark(gsph_handle h, int frames, gsph_bench_report *out);
  * handle's stream between its stages (frames then run without graphs).
  * gsph_stage_times waits for the stream and returns the mean device time (ms)
  * per frame since the previous call: {arrange, density, force, integrate};
- * density and force are one kernel launch each. */
+ * density and force run their TRA and SMS kernels side by side, and a frame's
+ * integration is part of its force stage. */
 gsph_status gsph_set_stage_timing(gsph_handle h, int enabled);
 gsph_status gsph_stage_times(gsph_handle h, float out[4]);
 
