@@ -1765,7 +1765,6 @@ gsph_status gsph_step_host_async(gsph_handle h, int frames, void *pos4, void *ve
                                   GSPH_FIELD_EVAL_VELOCITY};
     void *host[3] = {pos4, vel4, ev4};
     const size_t bytes = size_t(s.n) * sizeof(float4);
-    const bool split = s.in_parts(host);
     // upload: each array after its previous return copy (if any) is done; the
     // velocities behind the positions, beside the first frame's work on these
     for (int k = 0; k < 3; ++k) {
@@ -1788,6 +1787,7 @@ gsph_status gsph_step_host_async(gsph_handle h, int frames, void *pos4, void *ve
     // the last of them
     const bool graphs = s.graph_frames > 0 && frames >= s.graph_frames;
     if (frames > 0 && bytes && !graphs && !s.timing) {
+        const bool split = s.in_parts(host);   // (looked up beside the upload)
         if ((st = s.tick_host(true, frames == 1, host, split))) return st;
         for (int k = 1; k < frames; ++k)
             if ((st = s.tick_host(false, k == frames - 1, host, split))) return st;
