@@ -392,12 +392,12 @@ constexpr size_t kRowPrefetchCellBytes = size_t(64) << 20;
 // The blocks per SM decide, all of which run at once. A row per warp gives way
 // where units start to wait (5 per SM), three rows where some SMs have a fourth
 // block and the others three (9 to 11, where the single rows are ahead again), and
-// for good at a seventh (18). Force: the four lanes' blocks of 32 particles run at
-// most four to an SM without waiting. An SM runs 22 warps of the small build at
-// once and 32 of the general one: the general one is better from where the
-// small one needs a second wave until it needs one itself; from 34 to 40 units
-// both do, and the small one's is the fuller. Frames in CUDA graphs on 152 SMs,
-// the dam break, us (three runs, 0.1 to 0.5 apart):
+// for good at a seventh (18). Force: the four lanes are ahead to 4 units in graphs
+// and to 5 kernel by kernel, and the line keeps the latter. An SM runs 22 warps
+// of the small build at once and 32 of the general one: the general one is better
+// from where the small one needs a second wave until it needs one itself; from 34
+// to 40 units both do, and the small one's is the fuller. Frames in CUDA graphs on
+// 152 SMs, the dam break, us (three runs, 0.1 to 0.5 apart):
 //   units per SM            1.6   3.6   4.5   5.0   5.6   8.8   9.6  10.4  12.2  15.2  17.5  18.7
 //   density, row per warp  28.0  31.7  38.4  40.7  41.9  47.4  46.7  51.7  53.6  59.8  63.5  66.6
 //   density, three rows    31.4  34.4  40.9  38.8  38.7  44.3  50.3  51.8  54.3  56.3  58.1  69.0
@@ -411,10 +411,14 @@ constexpr size_t kRowPrefetchCellBytes = size_t(64) << 20;
 //   force, general         75.5  76.5  77.0  78.7  80.7  87.8  89.7  95.2  92.2  98.0  97.1 110.3
 // The same fluid in motion agrees (row per warp / three rows at 9.6 units 55.6 /
 // 59.2, at 12.2 58.2 / 57.7; four lanes / small at 4.0 37.7 / 36.6; small / general at
-// 22.7 83.0 / 80.6, at 38.1 95.4 / 99.3, at 42.2 105.7 / 103.4).
+// 22.7 83.0 / 80.6, at 38.1 95.4 / 99.3, at 42.2 105.7 / 103.4), and so do frames
+// launched kernel by kernel, but for the four lanes (four lanes / small at 4.0
+// 41.7 / 43.7, 4.5 43.3 / 44.8, 5.0 47.8 / 49.2, 5.6 49.7 / 49.2; row per warp / three
+// rows at 9.6 55.1 / 59.5, 12.2 62.9 / 62.7; small / general at 20.0 76.2 / 78.6, 21.3
+// 83.4 / 81.2, 36.1 95.6 / 96.0, 42.2 107.8 / 104.8).
 constexpr int kRowsMax1 = 5, kRowsAgain1 = 9, kRowsAgainMax1 = 11;
 constexpr int kRowsMax3 = 18;
-constexpr int kForceQuadMax = 4;
+constexpr int kForceQuadMax = 5;
 constexpr int kForceSmallMax = 21, kForceSmallAgain = 34, kForceSmallAgainMax = 40;
 // From how many units per SM a host step's force pass goes in parts
 // (System::force_downloading): a part costs launches and a tail, and has to be worth
