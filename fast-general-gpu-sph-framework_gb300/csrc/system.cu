@@ -110,6 +110,7 @@ struct System {
     // The passes take their units from queues that the cell scan resets. Set
     // by a stage call: the next one on the same grid resets its own (refill).
     bool density_spent = false, force_spent = false;
+    unsigned long long arranged_in = 0;   // the capture that holds gsph_arrange's launches
     uint64_t frames = 0;
 
     LaunchShape shape = kMaxShape;   // CTAs per SM of the density/force kernels
@@ -587,13 +588,18 @@ struct System {
         counts_dirty = false;
         density_spent = force_spent = false;
     }
+    // The capture the stream is in (0: none).
+    unsigned long long capture() const {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        unsigned long long id = 0;
+        cudaStreamGetCaptureInfo(stream, &status, &id);
+        return status == cudaStreamCaptureStatusNone ? 0 : id;
+    }
     // Before a stage call's pass: its queues (TRA and SMS, side by side) anew if
-    // an earlier call has used them up since the arrange, or if the launch is
-    // captured and may be replayed without one.
+    // an earlier call has used them up since the arrange, or if the arrange is not
+    // in the same capture and this launch may be replayed without it.
     void refill(int32_t Counters::*queue, bool &spent) {
-        cudaStreamCaptureStatus captured = cudaStreamCaptureStatusNone;
-        if (!spent) cudaStreamIsCapturing(stream, &captured);
-        if (spent || captured != cudaStreamCaptureStatusNone)
+        if (spent || capture() != arranged_in)
             cudaMemsetAsync(&(fr.ctr->*queue), 0, 2 * sizeof(int32_t), stream);
         spent = true;
     }
@@ -1383,6 +1389,7 @@ gsph_status gsph_arrange(gsph_handle h) {
     if (st) return st;
     System &s = h->sys;
     s.enqueue_arrange(s.cur);
+    s.arranged_in = s.capture();
     if ((st = s.check_launch())) return st;
     s.cur = 1 - s.cur;
     s.arranged = true;

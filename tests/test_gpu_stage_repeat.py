@@ -107,3 +107,33 @@ def test_a_captured_force_call_can_be_replayed(gsph, cuda_device):
     assert not np.array_equal(first, second)
     # (the captured launch walks the masks, the plain one after a copy-in scans)
     assert np.allclose(second, plain, rtol=1e-3, atol=1e-3 * np.abs(plain).max())
+
+
+def test_captured_stages_with_their_arrange_can_be_replayed(gsph, cuda_device):
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    p, pos = scene(gsph, "mixed, queued", sms)
+    fields = (gsph.FIELD_POSITION, gsph.FIELD_EVAL_VELOCITY, gsph.FIELD_ACCELERATION)
+    with gsph.HybridSystem(params=p, positions=pos) as h:
+        h.arrange()
+        h.density()
+        h.force()
+        ref = [h.copy_out(f) for f in fields]
+    with gsph.HybridSystem(params=p, positions=pos) as h:
+        stream = torch.cuda.ExternalStream(h.stream())
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.stream(stream):
+            graph.capture_begin(capture_error_mode="thread_local")
+            h.arrange()
+            h.density()
+            h.force()
+            graph.capture_end()
+            for _ in range(2):
+                graph.replay()
+        got = [h.copy_out(f) for f in fields]
+        h.density()   # and a plain call after them
+        h.force()
+        again = [h.copy_out(f) for f in fields]
+    for a, b, c in zip(ref, got, again):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+        assert np.array_equal(a.view(np.uint32), c.view(np.uint32))
