@@ -666,6 +666,18 @@ struct ClusterBox {
     int x0, x1, y0, y1, z0, z1;         // micro cells inside the cell, [0, 3]
 };
 
+// A position no farther than kFar, from where no squared distance overflows: a
+// particle outside the grid may be anywhere, and a cluster's box with it. (Box
+// widening, this and the position read again at the end: 3.94M dense particles
+// 20.3 -> 20.1 ms a host step, 64,000 498 -> 485 us; the box test given its own margin
+// instead 20.5 ms, stray clusters scanned apart 20.6.)
+__device__ __forceinline__ float4 on_scale(float4 p) {
+    p.x = fminf(fmaxf(p.x, -kFar), kFar);
+    p.y = fminf(fmaxf(p.y, -kFar), kFar);
+    p.z = fminf(fmaxf(p.z, -kFar), kFar);
+    return p;
+}
+
 __device__ __forceinline__ float warp_max(float v) {   // v >= 0
     return __uint_as_float(__reduce_max_sync(kFull, __float_as_uint(v)));
 }
@@ -683,9 +695,12 @@ __device__ __forceinline__ ClusterBox cluster_box(const float4 &p, uint32_t key)
     b.cx = 0.5f * (l[0] + h[0]);
     b.cy = 0.5f * (l[1] + h[1]);
     b.cz = 0.5f * (l[2] + h[2]);
-    b.ex = warp_max(fabsf(p.x - b.cx));
-    b.ey = warp_max(fabsf(p.y - b.cy));
-    b.ez = warp_max(fabsf(p.z - b.cz));
+    // wider by four roundings: a particle outside the grid, clamped into the cell,
+    // may stretch the box until its differences round by more than h
+    const float wider = 1.f + 4.f / 16777216.f;
+    b.ex = wider * warp_max(fabsf(p.x - b.cx));
+    b.ey = wider * warp_max(fabsf(p.y - b.cy));
+    b.ez = wider * warp_max(fabsf(p.z - b.cz));
     const uint32_t m = __reduce_or_sync(kFull, (1u << ((key >> 4) & 3u)) |
                                                    (16u << (key & 3u)) |
                                                    (256u << ((key >> 2) & 3u)));
@@ -825,7 +840,7 @@ __device__ __forceinline__ void cluster_stream(const Frame &f, const SceneGeom &
     const int nseg = cluster_segments(f, G, task, box, lane, ls.seg);
     const unsigned lt = lanemask_lt();
     // differences of coordinates round to 2^-24 of themselves, so 1e-5 of h^2
-    // covers the test's rounding
+    // covers the test's rounding (beside the box's own, see cluster_box)
     const float reach = h2 * 1.00001f;
     auto near = [&](const float4 &q) {
         const float ax = fmaxf(fabsf(q.x - box.cx) - box.ex, 0.f);
@@ -906,7 +921,7 @@ k_density_sms(Frame f, DevParams P) {
         const int cend = task.cell_begin + task.cell_particle_count;
         if (first >= cend) continue;   // warp-uniform
         const int self = min(first + i, cend - 1);
-        const float4 p = f.pos[self];
+        const float4 p = on_scale(f.pos[self]);
         const SceneGeom G = geom_of_cell(f.scenes, task.cellid);
         const ClusterBox box = cluster_box(p, f.key[self]);
         const float2 npx = make_float2(-p.x, -p.x);
@@ -1229,8 +1244,9 @@ k_force_tra_quad(Frame f, DevParams P, bool fresh) {
 // over the density pass's candidates. Bound by the FP32 pipe (66% busy with 3.94M
 // dense particles, 13.0 ms; most instructions of a pair step are packed and hold
 // it for two cycles) and, beside it, by the candidate tests. Three blocks per SM,
-// 80 registers: 244 bytes a thread are spilled and 120 loaded again (220 and 88
-// with artificial viscosity); at four blocks, 64 registers, the pass was slower
+// 80 registers: 228 bytes a thread are spilled and 92 loaded again (208 and 76
+// with artificial viscosity; the position is read again at the end, which saved
+// some); at four blocks, 64 registers, the pass was slower
 // (13.3 ms against 12.5, before the velocities' differences were taken per pair).
 // Each candidate pair is staged as four float4s (one 16-byte load per pair and
 // quantity group) and evaluated with packed FP32x2 arithmetic. Each term rounds as
@@ -1264,7 +1280,7 @@ k_force_sms(Frame f, DevParams P, int resident) {
         const int cend = task.cell_begin + task.cell_particle_count;
         if (first >= cend) continue;   // warp-uniform
         const int self = min(first + i, cend - 1);
-        const float4 p = f.pos[self];
+        const float4 p = on_scale(f.pos[self]);
         const float4 pev = f.ev[self];
         const SceneGeom G = geom_of_cell(f.scenes, task.cellid);
         const ClusterBox box = cluster_box(p, f.key[self]);
@@ -1398,7 +1414,7 @@ k_force_sms(Frame f, DevParams P, int resident) {
             a.gy = -s[7];
             a.gz = -s[8];
             a.lap = s[9];
-            write_force(f, P, self, p, pev, G, a, true);
+            write_force(f, P, self, f.pos[self], pev, G, a, true);
         }
     }
 }
