@@ -647,7 +647,7 @@ k_density_tra_rows(Frame f, DevParams P) {
 // arithmetic is bound by the FP32 pipe and wants small clusters, the testing
 // by issue slots and wants large ones, and small scenes want many units:
 // force, 3.94M particles 14.0 / 12.5 ms and 64,000 particles 260 / 277 us at
-// C = 8 / 16 (with two packed operations a pair less than now: 13.0 ms at 16);
+// C = 8 / 16 (with two packed operations a pair less than now: 12.8 ms at 16);
 // density 6.8 / 5.2 / 4.8 ms and 146 / 154 / 165 us at 8 / 16 / 32. Whole tasks
 // without the box test took 16.3 ms and 690 us (force), 6.7 ms and 230 us
 // (density).
@@ -1241,13 +1241,13 @@ k_force_tra_quad(Frame f, DevParams P, bool fresh) {
 
 // -------------------------------------------------------------- force SMS --
 // One cluster of kForceCluster particles per warp (force_kernels.cu:830-1054),
-// over the density pass's candidates. Bound by the FP32 pipe (66% busy with 3.94M
-// dense particles, 13.0 ms; most instructions of a pair step are packed and hold
+// over the density pass's candidates. Bound by the FP32 pipe (67% busy with 3.94M
+// dense particles, 12.8 ms; most instructions of a pair step are packed and hold
 // it for two cycles) and, beside it, by the candidate tests. Three blocks per SM,
 // 80 registers: 228 bytes a thread are spilled and 92 loaded again (208 and 76
 // with artificial viscosity; the position is read again at the end, which saved
-// some); at four blocks, 64 registers, the pass was slower
-// (13.3 ms against 12.5, before the velocities' differences were taken per pair).
+// some); at four blocks, 64 registers, the pass was slower (13.3 ms against 12.5,
+// before the velocities' differences were taken per pair).
 // Each candidate pair is staged as four float4s (one 16-byte load per pair and
 // quantity group) and evaluated with packed FP32x2 arithmetic. Each term rounds as
 // the reference's scalar expression; the two halves of every accumulator and then
